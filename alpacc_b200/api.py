@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from dataclasses import dataclass
 from typing import List, Optional, Sequence, Tuple, Union
 
@@ -32,6 +33,61 @@ class AlpError(RuntimeError):
         self.code = code
 
 
+_ALLOC_OFF, _ALLOC_VALID = 5, 6
+_ALLOC_FN = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_int64, ctypes.POINTER(ctypes.c_void_p))
+_wanted = threading.local()  # .outputs: the _Outputs of this thread's call
+
+
+class _Outputs:
+    """The output tensors of one native call, allocated on the current stream when
+    the call knows their length (alp_set_output_alloc): the kernels then write the
+    caller's tensors and nothing is copied."""
+
+    def __init__(self, g: "Grammar", dtypes, n_docs: int = 0):
+        self.g, self.dtypes, self.n_docs = g, dtypes, n_docs
+        self.tensors, self.off, self.valid, self.error = None, None, None, None
+
+    def make(self, n: int, ptrs=None) -> None:
+        torch = _torch()
+        dev = self.g.device
+        self.tensors = [torch.empty(n, dtype=dt, device=dev) for dt in self.dtypes]
+        if self.n_docs:
+            self.off = torch.empty(self.n_docs + 1, dtype=torch.int64, device=dev)
+            self.valid = torch.empty(self.n_docs, dtype=torch.uint8, device=dev)
+        if ptrs is not None:
+            for i, t in enumerate(self.tensors):
+                ptrs[i] = t.data_ptr()
+            if self.n_docs:
+                ptrs[_ALLOC_OFF], ptrs[_ALLOC_VALID] = self.off.data_ptr(), self.valid.data_ptr()
+
+    def __enter__(self) -> "_Outputs":
+        _wanted.outputs = self
+        native().alp_set_output_alloc(self.g.h, _alloc_outputs, None)
+        return self
+
+    def __exit__(self, *exc) -> None:
+        native().alp_set_output_alloc(self.g.h, _NO_ALLOC, None)
+        _wanted.outputs = None
+
+    def check(self, rc: int) -> None:
+        if self.error is not None:
+            raise self.error
+        if rc != ALP_OK:
+            self.g._err(rc)
+
+
+@_ALLOC_FN
+def _alloc_outputs(user, n, ptrs):
+    out = _wanted.outputs
+    try:
+        out.make(n, ptrs)
+        return 0
+    except BaseException as e:  # raised again by check(), in the caller
+        out.error = e
+        return 1
+
+
+_NO_ALLOC = _ALLOC_FN(0)
 _lib = None
 
 
@@ -81,6 +137,7 @@ def native() -> ctypes.CDLL:
         L.alp_parse_graph_destroy.argtypes = [vp]
         L.alp_parse_graph_destroy.restype = None
         L.alp_check_bounded_wait.argtypes = [vp]
+        L.alp_set_output_alloc.argtypes = [vp, _ALLOC_FN, vp]
         L.alp_tune_parse.argtypes = [vp, vp, i64, i32, ctypes.c_char_p, ctypes.c_size_t]
         L.alp_tune_get.argtypes = [vp, P(i32), i32]
         L.alp_tune_set.argtypes = [vp, P(i32), i32]
@@ -201,17 +258,12 @@ class Grammar:
         self._stream()
         pt, ps, pe = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
         n, valid = ctypes.c_int64(0), ctypes.c_int(0)
-        rc = native().alp_lex(self.h, ctypes.c_void_p(x.data_ptr()), x.numel(), ctypes.byref(pt), ctypes.byref(ps),
-                              ctypes.byref(pe), ctypes.byref(n), ctypes.byref(valid))
-        if rc != ALP_OK:
-            self._err(rc)
+        with _Outputs(self, (torch.int32, torch.int64, torch.int64)) as out:
+            out.check(native().alp_lex(self.h, ctypes.c_void_p(x.data_ptr()), x.numel(), ctypes.byref(pt),
+                                       ctypes.byref(ps), ctypes.byref(pe), ctypes.byref(n), ctypes.byref(valid)))
         if not valid.value:
             return None
-        k = n.value
-        term = _wrap(self.h, pt.value or 0, k, torch.int32, self.device)
-        start = _wrap(self.h, ps.value or 0, k, torch.int64, self.device)
-        end = _wrap(self.h, pe.value or 0, k, torch.int64, self.device)
-        return term, start, end
+        return tuple(out.tensors)
 
     def lex(self, data) -> Optional[List[Tuple[str, Tuple[int, int]]]]:
         r = self.lex_int(data)
@@ -268,13 +320,9 @@ class Grammar:
         return term[:k], start[:k], end[:k]
 
     # ----------------------------------------------------------------- parser
-    def _tree(self, pp, pt, pk, ps, pe, n) -> Tree:
+    def _tree_outputs(self, n_docs: int = 0) -> _Outputs:
         torch = _torch()
-        return Tree(_wrap(self.h, pp.value or 0, n, torch.int64, self.device),
-                    _wrap(self.h, pt.value or 0, n, torch.int32, self.device),
-                    _wrap(self.h, pk.value or 0, n, torch.uint8, self.device),
-                    _wrap(self.h, ps.value or 0, n, torch.int64, self.device),
-                    _wrap(self.h, pe.value or 0, n, torch.int64, self.device))
+        return _Outputs(self, (torch.int64, torch.int32, torch.uint8, torch.int64, torch.int64), n_docs)
 
     def parse_int(self, data) -> Optional[Tree]:
         """Bytes -> preorder tree (parent, tag, kind, start, end), or None."""
@@ -282,13 +330,12 @@ class Grammar:
         self._stream()
         ptrs = [ctypes.c_void_p() for _ in range(5)]
         n, valid = ctypes.c_int64(0), ctypes.c_int(0)
-        rc = native().alp_parse(self.h, ctypes.c_void_p(x.data_ptr()), x.numel(), *[ctypes.byref(p) for p in ptrs],
-                                ctypes.byref(n), ctypes.byref(valid))
-        if rc != ALP_OK:
-            self._err(rc)
+        with self._tree_outputs() as out:
+            out.check(native().alp_parse(self.h, ctypes.c_void_p(x.data_ptr()), x.numel(),
+                                         *[ctypes.byref(p) for p in ptrs], ctypes.byref(n), ctypes.byref(valid)))
         if not valid.value:
             return None
-        return self._tree(*ptrs, n.value)
+        return Tree(*out.tensors)
 
     def parse(self, data):
         """Named tree: a list of (parent, ('terminal', name, (start, end)) |
@@ -315,14 +362,14 @@ class Grammar:
         self._stream()
         ptrs = [ctypes.c_void_p() for _ in range(5)]
         n, valid = ctypes.c_int64(0), ctypes.c_int(0)
-        rc = native().alp_parse_tokens(self.h, ctypes.c_void_p(term.data_ptr()), ctypes.c_void_p(start.data_ptr()),
-                                       ctypes.c_void_p(end.data_ptr()), term.numel(),
-                                       *[ctypes.byref(p) for p in ptrs], ctypes.byref(n), ctypes.byref(valid))
-        if rc != ALP_OK:
-            self._err(rc)
+        with self._tree_outputs() as out:
+            out.check(native().alp_parse_tokens(self.h, ctypes.c_void_p(term.data_ptr()),
+                                                ctypes.c_void_p(start.data_ptr()), ctypes.c_void_p(end.data_ptr()),
+                                                term.numel(), *[ctypes.byref(p) for p in ptrs], ctypes.byref(n),
+                                                ctypes.byref(valid)))
         if not valid.value:
             return None
-        return self._tree(*ptrs, n.value)
+        return Tree(*out.tensors)
 
     def pre_productions_int(self, term) -> Optional["torch.Tensor"]:
         torch = _torch()
@@ -381,16 +428,10 @@ class Grammar:
         self._stream()
         ptrs = [ctypes.c_void_p() for _ in range(5)]
         total = ctypes.c_int64(0)
-        rc = native().alp_lex_batch(self.h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(off.data_ptr()), nd,
-                                    *[ctypes.byref(p) for p in ptrs], ctypes.byref(total))
-        if rc != ALP_OK:
-            self._err(rc)
-        k = total.value
-        return (_wrap(self.h, ptrs[0].value or 0, k, torch.int32, self.device),
-                _wrap(self.h, ptrs[1].value or 0, k, torch.int64, self.device),
-                _wrap(self.h, ptrs[2].value or 0, k, torch.int64, self.device),
-                _wrap(self.h, ptrs[3].value or 0, nd + 1, torch.int64, self.device),
-                _wrap(self.h, ptrs[4].value or 0, nd, torch.uint8, self.device))
+        with _Outputs(self, (torch.int32, torch.int64, torch.int64), nd) as out:
+            out.check(native().alp_lex_batch(self.h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(off.data_ptr()),
+                                             nd, *[ctypes.byref(p) for p in ptrs], ctypes.byref(total)))
+        return tuple(out.tensors) + (out.off, out.valid)
 
     # ---------------------------------------------------------------- tuning
     @staticmethod
@@ -462,14 +503,10 @@ class Grammar:
         self._stream()
         ptrs = [ctypes.c_void_p() for _ in range(7)]
         total = ctypes.c_int64(0)
-        rc = native().alp_parse_batch(self.h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(off.data_ptr()), nd,
-                                      *[ctypes.byref(p) for p in ptrs], ctypes.byref(total))
-        if rc != ALP_OK:
-            self._err(rc)
-        k = total.value
-        tree = self._tree(*ptrs[:5], k)
-        return (tree, _wrap(self.h, ptrs[5].value or 0, nd + 1, torch.int64, self.device),
-                _wrap(self.h, ptrs[6].value or 0, nd, torch.uint8, self.device))
+        with self._tree_outputs(nd) as out:
+            out.check(native().alp_parse_batch(self.h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(off.data_ptr()),
+                                               nd, *[ctypes.byref(p) for p in ptrs], ctypes.byref(total)))
+        return Tree(*out.tensors), out.off, out.valid
 
 
     def parse_batch_host(self, data, offsets, cap: Optional[int] = None):

@@ -119,6 +119,12 @@ struct alp_ctx {
     int32_t* h_ring = nullptr;
     cudaEvent_t ev_ring[RING_SLOTS] = {};
     HostPool* pool = nullptr;
+    // when set (alp_set_output_alloc): the caller's allocator for the outputs of alp_lex,
+    // alp_parse, alp_parse_tokens and the batch entry points
+    alp_alloc_fn alloc_fn = nullptr;
+    void* alloc_user = nullptr;
+    void* alloc_off = nullptr;    // of a batch: where the allocator wants the documents' offsets
+    void* alloc_valid = nullptr;  // and their validity (null: left in the context's buffers)
     long long last_h2d = 0, last_d2h = 0;  // data bytes the last host-buffer call moved
     // when set (pinned, in h_stage): the lexer copies the validity of document 0
     // here in the same wait as its token count, which saves the caller a wait of its own
@@ -293,6 +299,28 @@ int grow(alp_ctx* ctx, DevBuf& b, size_t bytes) {
     CK(cudaMalloc(&b.p, want));
     ++ctx->dev_allocs;
     b.bytes = want;
+    return ALP_OK;
+}
+
+// Outputs of n elements each from the caller's allocator (`count` pointers).
+int alloc_outputs(alp_ctx* ctx, long long n, void** ptrs, int count) {
+    void* p[ALP_ALLOC_PTRS] = {};
+    if (ctx->alloc_fn(ctx->alloc_user, n, p)) return fail(ctx, ALP_ERR_CUDA, "the output allocator failed");
+    for (int i = 0; i < count; ++i) {
+        if (n > 0 && !p[i]) return fail(ctx, ALP_ERR_ARG, "the output allocator gave no buffer");
+        ptrs[i] = p[i];
+    }
+    ctx->alloc_off = p[ALP_ALLOC_OFF];
+    ctx->alloc_valid = p[ALP_ALLOC_VALID];
+    return ALP_OK;
+}
+
+// A batch's offsets and validity into the allocator's buffers (stream-ordered).
+int batch_out(alp_ctx* ctx, const void* off, const void* valid, long long nd) {
+    if (!ctx->alloc_fn) return ALP_OK;
+    if (ctx->alloc_off)
+        CK(cudaMemcpyAsync(ctx->alloc_off, off, (size_t)(nd + 1) * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+    if (ctx->alloc_valid) CK(cudaMemcpyAsync(ctx->alloc_valid, valid, (size_t)nd, cudaMemcpyDeviceToDevice, ctx->stream));
     return ALP_OK;
 }
 
@@ -756,7 +784,7 @@ int lex3_tiles(alp_ctx* ctx, Lex3Run& r) {
     unsigned long long* ccs = reinterpret_cast<unsigned long long*>(r.base + r.o_ccs);
     lex3_tile_reduce_kernel<<<(unsigned)lchunks, LT_CHUNK, 0, ctx->stream>>>(r.a.tile_cs, r.tiles, ccs);
     CK(cudaGetLastError());
-    lex3_tile_scan_kernel<<<(unsigned)lchunks, LT_CHUNK, 0, ctx->stream>>>(r.a.tile_cs, r.tiles, ccs);
+    lex3_tile_scan_kernel<<<(unsigned)lchunks, LT_CHUNK, 0, ctx->stream>>>(r.a.tile_cs, r.tiles, ccs, r.a.res);
     CK(cudaGetLastError());
     return ALP_OK;
 }
@@ -770,8 +798,10 @@ int lex3_emit(alp_ctx* ctx, Lex3Run& r, bool tiles_done = false) {
     CK(cudaFuncSetAttribute(k5, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     if ((rc = lex3_grid(ctx, r, (const void*)k5, LX_THREADS, ctx->l3_emit_smem, r.tiles, &g5))) return rc;
     mark(ctx, "start");
-    if (!tiles_done && (rc = lex3_tiles(ctx, r))) return rc;
-    mark(ctx, "lex3_tile_reduce+lex3_tile_scan");
+    if (!tiles_done) {
+        if ((rc = lex3_tiles(ctx, r))) return rc;
+        mark(ctx, "lex3_tile_reduce+lex3_tile_scan");
+    }
     k5<<<g5, LX_THREADS, ctx->l3_emit_smem, ctx->stream>>>(r.a, r.sg);
     CK(cudaGetLastError());
     mark(ctx, "lex3_emit_kernel");
@@ -853,6 +883,43 @@ int lex3_run(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long* d_
     }
     if ((rc = lex3_states(ctx, r))) return rc;
     return lex3_tok<TermT, PosT>(ctx, r, total);
+}
+
+// The lexer API layout into buffers from the caller's allocator: the token total
+// (and one document's verdict) is known after the tile scan, before any token is
+// written, so the outputs are allocated at their exact size and the token pass
+// writes them once.  One document that is rejected gets no outputs.
+int lex3_run_alloc(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long* d_off, long long nd,
+                   uint8_t* valid, void** ptrs, long long* total, int* accepted) {
+    Lex3Run r;
+    int rc;
+    *total = 0;
+    if ((rc = lex3_prepare(ctx, d_in, n, d_off, nd, 0, nullptr, nullptr, nullptr, 0, valid, r)) ||
+        (rc = lex3_front(ctx, r)))
+        return rc;
+    mark(ctx, "start");
+    if ((rc = lex3_tiles(ctx, r))) return rc;
+    mark(ctx, "lex3_tile_reduce+lex3_tile_scan");
+    CK(cudaMemcpyAsync(ctx->h_res, r.a.res, sizeof(AlpResult), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (ctx->h_res->error & ALP_DEV_ERR_TIMEOUT) return fail(ctx, ALP_ERR_TIMEOUT, "lexer look-back timed out");
+    const long long m = ctx->h_res->aux[6];
+    ctx->last_tokens = m;
+    if (nd == 1) {
+        *accepted = ctx->h_res->aux[7] ? 1 : 0;
+        if (!*accepted) return ALP_OK;
+    }
+    if ((rc = alloc_outputs(ctx, m, ptrs, 3))) return rc;
+    r.a.out_term = ptrs[0];
+    r.a.out_start = ptrs[1];
+    r.a.out_end = ptrs[2];
+    r.a.cap = m;
+    if ((rc = lex3_emit<uint32_t, int64_t>(ctx, r, true)) || (rc = batch_out(ctx, r.sg.tok_off, valid, nd))) return rc;
+    CK(cudaMemcpyAsync(ctx->h_res, r.a.res, sizeof(AlpResult), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (ctx->h_res->error & ALP_DEV_ERR_CAPACITY) return fail(ctx, ALP_ERR_CUDA, "token counts disagree");
+    *total = m;
+    return ALP_OK;
 }
 
 // Segmented lexer over documents at d_off[0..nd] (device).  sentinels: the
@@ -944,9 +1011,18 @@ int put_doc_off(alp_ctx* ctx, long long n) {
 // documents land in tmp[T_NODEOFF].
 // Output buffers for N nodes (context-owned when ctx_out) and the node and
 // bracket intermediates for N nodes and K kept brackets.
-int parse_buffers(alp_ctx* ctx, ParseOut* o, int ctx_out, long long N, long long K, ParseArgs& a) {
+// `exact`: N is the node count, for which a caller's allocator can be asked.
+int parse_buffers(alp_ctx* ctx, ParseOut* o, int ctx_out, long long N, long long K, ParseArgs& a, bool exact = true) {
     int rc;
-    if (ctx_out) {
+    if (ctx_out && ctx->alloc_fn && exact) {
+        void* p[5] = {};
+        if ((rc = alloc_outputs(ctx, N, p, 5))) return rc;
+        o->parent = (int64_t*)p[0];
+        o->tag = (uint32_t*)p[1];
+        o->kind = (uint8_t*)p[2];
+        o->start = (int64_t*)p[3];
+        o->end = (int64_t*)p[4];
+    } else if (ctx_out) {
         if ((rc = grow(ctx, ctx->out[3], N * 8 + 8)) || (rc = grow(ctx, ctx->out[4], N * 4 + 8)) ||
             (rc = grow(ctx, ctx->out[5], N + 8)) || (rc = grow(ctx, ctx->out[6], N * 8 + 8)) ||
             (rc = grow(ctx, ctx->out[7], N * 8 + 8)))
@@ -1065,7 +1141,8 @@ int parse_positions(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, Pa
     long long N = 0, B = 0, K = 0;
     const bool fits32 = (unsigned long long)L * (unsigned long long)(ctx->ph.max_prods + 1) < (1ull << 32) &&
                         (unsigned long long)L * (unsigned long long)(ctx->ph.max_brackets + 1) < (1ull << 32);
-    if (!ctx->tune.parse_split && fits32 && ctx->est_nodes > 0) {
+    const bool fused = !ctx->tune.parse_split && fits32 && ctx->est_nodes > 0;
+    if (fused) {
         // ---- fused: capacities from the last parse, exact sizes on a second run if short
         const void* fn = fused_expand_for(ctx->pt.q, ctx->pt.k);
         unsigned g = 1;
@@ -1080,7 +1157,7 @@ int parse_positions(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, Pa
         long long capN = ctx_out ? (long long)(ctx->est_nodes * (double)L * 1.01) + 4096 : cap;
         long long capK = (long long)(ctx->est_kept * (double)L * 1.01) + 4096;
         for (int attempt = 0; attempt < 2; ++attempt) {
-            if ((rc = parse_buffers(ctx, o, ctx_out, capN, capK, a))) return rc;
+            if ((rc = parse_buffers(ctx, o, ctx_out, capN, capK, a, false))) return rc;
             CK(cudaMemsetAsync(lb, 0, 16 + 4 * (size_t)tiles, ctx->stream));  // ticket, look-back flags
             mark(ctx, "start");
             {
@@ -1214,6 +1291,17 @@ int parse_positions(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, Pa
         if ((rc = run_ple(ctx, a.dsbuf, K, a.brbuf, nullptr, T_B_TMIN, a.br_off, nd, dvalid, d_res))) return rc;
     }
     if (h_valid0) CK(cudaMemcpyAsync(h_valid0, dvalid, 1, cudaMemcpyDeviceToHost, ctx->stream));
+    if (fused && ctx_out && ctx->alloc_fn) {
+        // written at estimated capacities: copied into the allocator's buffers
+        void* p[5] = {};
+        if ((rc = alloc_outputs(ctx, N, p, 5))) return rc;
+        const void* src[5] = {o->parent, o->tag, o->kind, o->start, o->end};
+        const size_t w[5] = {8, 4, 1, 8, 8};
+        for (int i = 0; i < 5 && N > 0; ++i)
+            CK(cudaMemcpyAsync(p[i], src[i], (size_t)N * w[i], cudaMemcpyDeviceToDevice, ctx->stream));
+        *o = ParseOut{(int64_t*)p[0], (uint32_t*)p[1], (uint8_t*)p[2], (int64_t*)p[3], (int64_t*)p[4]};
+    }
+    if (ctx_out && (rc = batch_out(ctx, a.node_off, dvalid, nd))) return rc;
     if ((rc = read_result(ctx, d_res))) return rc;
     *n_node = N;
     return ALP_OK;
@@ -2035,12 +2123,57 @@ int alp_lex_noalloc(alp_ctx* ctx, const uint8_t* d_in, int64_t n, uint32_t* d_te
     return ALP_OK;
 }
 
+// The lexer's outputs where they lie in the context's buffers, or (with an output
+// allocator, on the paths that count while they write) copied into the caller's.
+static int tokens_out(alp_ctx* ctx, long long m, uint32_t** d_term, int64_t** d_start, int64_t** d_end) {
+    *d_term = (uint32_t*)ctx->out[0].p;
+    *d_start = (int64_t*)ctx->out[1].p;
+    *d_end = (int64_t*)ctx->out[2].p;
+    if (!ctx->alloc_fn) return ALP_OK;
+    void* p[3] = {};
+    int rc;
+    if ((rc = alloc_outputs(ctx, m, p, 3))) return rc;
+    if (m) {
+        CK(cudaMemcpyAsync(p[0], *d_term, (size_t)m * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+        CK(cudaMemcpyAsync(p[1], *d_start, (size_t)m * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+        CK(cudaMemcpyAsync(p[2], *d_end, (size_t)m * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+    }
+    *d_term = (uint32_t*)p[0];
+    *d_start = (int64_t*)p[1];
+    *d_end = (int64_t*)p[2];
+    return ALP_OK;
+}
+
+int alp_set_output_alloc(alp_ctx* ctx, alp_alloc_fn fn, void* user) {
+    if (!ctx) return ALP_ERR_ARG;
+    ctx->alloc_fn = fn;
+    ctx->alloc_user = user;
+    return ALP_OK;
+}
+
 int alp_lex(alp_ctx* ctx, const uint8_t* d_in, int64_t n, uint32_t** d_term, int64_t** d_start,
             int64_t** d_end, int64_t* n_tok, int* valid) {
     int rc = check_in(ctx, d_in, n, true);
     if (rc) return rc;
     if (!d_term || !d_start || !d_end || !n_tok || !valid) return fail(ctx, ALP_ERR_ARG, "null output");
     CK(cudaSetDevice(ctx->device));
+    if (ctx->alloc_fn && ctx->lex3 && ctx->tune.lex_split && n > 0) {
+        void* p[3] = {};
+        long long total = 0;
+        *n_tok = 0;
+        *valid = 0;
+        if ((rc = grow(ctx, ctx->tmp[T_DVALID], 16)) || (rc = grow(ctx, ctx->tmp[T_TOKOFF], 16)) ||
+            (rc = put_doc_off(ctx, n)) ||
+            (rc = lex3_run_alloc(ctx, d_in, n, (const long long*)ctx->tmp[T_DOCOFF].p, 1,
+                                 (uint8_t*)ctx->tmp[T_DVALID].p, p, &total, valid)))
+            return rc;
+        *n_tok = total;
+        *d_term = (uint32_t*)p[0];
+        *d_start = (int64_t*)p[1];
+        *d_end = (int64_t*)p[2];
+        return ALP_OK;
+    }
     int64_t cap = n / 2 + 1024;
     for (int attempt = 0; attempt < 2; ++attempt) {
         if ((rc = grow(ctx, ctx->out[0], cap * 4)) || (rc = grow(ctx, ctx->out[1], cap * 8)) ||
@@ -2053,10 +2186,7 @@ int alp_lex(alp_ctx* ctx, const uint8_t* d_in, int64_t n, uint32_t** d_term, int
         cap = *n_tok + 1;
     }
     if (rc) return rc;
-    *d_term = (uint32_t*)ctx->out[0].p;
-    *d_start = (int64_t*)ctx->out[1].p;
-    *d_end = (int64_t*)ctx->out[2].p;
-    return ALP_OK;
+    return tokens_out(ctx, *valid ? *n_tok : 0, d_term, d_start, d_end);
 }
 
 int alp_lex_host(alp_ctx* ctx, const uint8_t* h_in, int64_t n, uint32_t* h_term, int64_t* h_start,
@@ -2986,9 +3116,10 @@ int alp_parse_tokens(alp_ctx* ctx, const uint32_t* d_term, const int64_t* d_tsta
     ParseOut o{};
     uint8_t* dvalid = (uint8_t*)ctx->tmp[T_DVALID].p;
     int64_t N = 0;
-    rc = parse_positions(ctx, m + 2, 1, dvalid, &o, 0, 1, &N, 1);
+    uint8_t* hv = reinterpret_cast<uint8_t*>(ctx->h_stage) + 200;
+    rc = parse_positions(ctx, m + 2, 1, dvalid, &o, 0, 1, &N, 1, hv);
     if (rc) return rc;
-    if ((rc = read_valid0(ctx, dvalid, valid))) return rc;
+    *valid = hv[0] ? 1 : 0;
     *n_node = *valid ? N : 0;
     *d_parent = o.parent;
     *d_tag = o.tag;
@@ -3414,6 +3545,23 @@ int alp_lex_batch(alp_ctx* ctx, const uint8_t* d_in, const int64_t* d_off, int64
     n = ctx->h_stage[0];
     int rc = check_in(ctx, d_in, n, true);
     if (rc) return rc;
+    if (ctx->alloc_fn && ctx->lex3 && ctx->tune.lex_split && n > 0) {
+        void* p[3] = {};
+        long long total = 0;
+        int accepted = 0;
+        if ((rc = grow(ctx, ctx->tmp[T_DVALID], (size_t)n_docs + 16)) ||
+            (rc = grow(ctx, ctx->tmp[T_TOKOFF], (size_t)(n_docs + 1) * 8)) ||
+            (rc = lex3_run_alloc(ctx, d_in, n, (const long long*)d_off, n_docs, (uint8_t*)ctx->tmp[T_DVALID].p, p,
+                                 &total, &accepted)))
+            return rc;
+        *d_term = (uint32_t*)p[0];
+        *d_start = (int64_t*)p[1];
+        *d_end = (int64_t*)p[2];
+        *d_tok_off = (int64_t*)ctx->tmp[T_TOKOFF].p;
+        *d_valid = (uint8_t*)ctx->tmp[T_DVALID].p;
+        *n_tok_total = total;
+        return ALP_OK;
+    }
     if ((rc = grow(ctx, ctx->out[0], (size_t)n * 4 + 16)) || (rc = grow(ctx, ctx->out[1], (size_t)n * 8 + 16)) ||
         (rc = grow(ctx, ctx->out[2], (size_t)n * 8 + 16)) || (rc = grow(ctx, ctx->tmp[T_DVALID], (size_t)n_docs + 16)))
         return rc;
@@ -3422,9 +3570,10 @@ int alp_lex_batch(alp_ctx* ctx, const uint8_t* d_in, const int64_t* d_off, int64
                                     (int64_t*)ctx->out[1].p, (int64_t*)ctx->out[2].p, n + 1,
                                     (uint8_t*)ctx->tmp[T_DVALID].p, &total);
     if (rc) return rc;
-    *d_term = (uint32_t*)ctx->out[0].p;
-    *d_start = (int64_t*)ctx->out[1].p;
-    *d_end = (int64_t*)ctx->out[2].p;
+    if ((rc = tokens_out(ctx, total, d_term, d_start, d_end)) ||
+        (rc = batch_out(ctx, ctx->tmp[T_TOKOFF].p, ctx->tmp[T_DVALID].p, n_docs)))
+        return rc;
+    if (ctx->alloc_fn) CK(cudaStreamSynchronize(ctx->stream));
     *d_tok_off = (int64_t*)ctx->tmp[T_TOKOFF].p;
     *d_valid = (uint8_t*)ctx->tmp[T_DVALID].p;
     *n_tok_total = total;

@@ -395,11 +395,13 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
 // ---- kernel 3: token counts -------------------------------------------------
 
 // Tokens ending in bytes in[0, lim) from state st, with document heads and
-// last bytes; *lastoff = offset of the last token start or LX_NOOFF.  A
-// compact loop: only chunks at document boundaries or the input's end.
+// last bytes; *lastoff = offset of the last token start or LX_NOOFF, *endinfo
+// = tokinfo of the state after the last document end in the chunk (kept
+// without one).  A compact loop: only chunks at document boundaries or the
+// input's end.
 __device__ __forceinline__ uint32_t lx_count_slow(const uint8_t* in, int lim, uint32_t st, uint32_t head,
                                                   uint32_t last, const uint16_t* s_ent, const uint32_t* s_tok,
-                                                  uint32_t* lastoff) {
+                                                  uint32_t* lastoff, uint32_t* endinfo) {
     uint32_t cnt = 0, lo = LX_NOOFF;
 #pragma unroll 1
     for (int j = 0; j < lim; ++j) {
@@ -409,7 +411,10 @@ __device__ __forceinline__ uint32_t lx_count_slow(const uint8_t* in, int lim, ui
             cnt += (e >> 6) & 1u;
             if (e & LX_START) lo = (uint32_t)j;
             st = e & LX_NEXT;
-            if (((last >> j) & 1u) && !(s_tok[st] & TOK_IGNORE)) ++cnt;
+            if ((last >> j) & 1u) {
+                *endinfo = s_tok[st];
+                if (!(s_tok[st] & TOK_IGNORE)) ++cnt;
+            }
         }
     }
     *lastoff = lo;
@@ -482,13 +487,16 @@ __global__ void __launch_bounds__(LX_THREADS, 6) lex3_count_kernel(Lex3Args a, L
                 }
                 *reinterpret_cast<uint32_t*>(a.chunk_c + c) = (ca | (oa << 8)) | ((cb | (ob << 8)) << 16);
             } else {
-                ca = lx_count_slow(a.in + my, min(lim, LX_CHUNK), a.chunk_s[c], ha, la, s_ent, s_tok, &oa);
+                uint32_t ei = 0;
+                ca = lx_count_slow(a.in + my, min(lim, LX_CHUNK), a.chunk_s[c], ha, la, s_ent, s_tok, &oa, &ei);
                 a.chunk_c[c] = (uint16_t)(ca | (oa << 8));
                 if (lim > LX_CHUNK) {
                     cb = lx_count_slow(a.in + my + LX_CHUNK, lim - LX_CHUNK, a.chunk_s[c + 1], hb, lb, s_ent, s_tok,
-                                       &ob);
+                                       &ob, &ei);
                     a.chunk_c[c + 1] = (uint16_t)(cb | (ob << 8));
                 }
+                // one document: accepted or not, known before its tokens are written
+                if (sg.n_docs == 1 && (la | lb)) a.res->aux[7] = (ei & TOK_ACCEPT) ? 1 : 0;
             }
             cnt = ca + cb;
             lastp = ob != LX_NOOFF ? (uint32_t)(my + LX_CHUNK + ob)
@@ -544,7 +552,7 @@ __global__ void __launch_bounds__(LT_CHUNK) lex3_tile_reduce_kernel(const unsign
 }
 
 __global__ void __launch_bounds__(LT_CHUNK) lex3_tile_scan_kernel(unsigned long long* tile_cs, long long T,
-                                                                  const unsigned long long* chunk_cs) {
+                                                                  const unsigned long long* chunk_cs, AlpResult* res) {
     __shared__ uint32_t s_c[LT_CHUNK / 32], s_p[LT_CHUNK / 32];
     __shared__ uint32_t s_cc, s_cp;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -583,6 +591,7 @@ __global__ void __launch_bounds__(LT_CHUNK) lex3_tile_scan_kernel(unsigned long 
     const uint32_t rc = s_cc + s_c[warp] + ec;
     uint32_t rp = ep != ALP_NONE32 ? ep : (s_p[warp] != ALP_NONE32 ? s_p[warp] : s_cp);
     if (i < T) tile_cs[i] = ((unsigned long long)rc << 32) | rp;
+    if (i == T - 1) res->aux[6] = (long long)rc + c;  // all tokens
 }
 
 // ---- kernel 5: tokens ---------------------------------------------------------
@@ -996,7 +1005,8 @@ __global__ void __launch_bounds__(LX_THREADS, 5) lex3_tok_kernel(Lex3Args a, Lex
             if (smask) lastp = (uint32_t)(my + 31 - __clz(smask));
         } else if (lim > 0) {
             uint32_t lo;
-            cnt = lx_count_slow(a.in + my, lim, s0, head, last, s_ent, s_tok, &lo);
+            uint32_t ei = 0;
+            cnt = lx_count_slow(a.in + my, lim, s0, head, last, s_ent, s_tok, &lo, &ei);
             if (lo != LX_NOOFF) lastp = (uint32_t)(my + lo);
         }
 

@@ -111,6 +111,20 @@ int alp_tune_shapes(int32_t* out, int n);
  * stream and wait for it; lets bindings move context-owned outputs. */
 int alp_memcpy(alp_ctx* ctx, void* dst, const void* src, size_t bytes);
 
+/* Outputs in the caller's memory at their exact size.  With an allocator set,
+ * alp_lex, alp_parse, alp_parse_tokens, alp_pre_productions and the two batch
+ * entry points call it once, from the calling thread, when the number of tokens
+ * or nodes `n` is known, write the outputs to its buffers (device memory) and
+ * return those pointers: ptrs[0..2] term, start, end or ptrs[0..4] parent, tag,
+ * kind, start, end, of n elements each; a batch also copies its n_docs + 1
+ * offsets to ptrs[ALP_ALLOC_OFF] and its validity to ptrs[ALP_ALLOC_VALID] where
+ * these are set (they are null on entry).  A nonzero return ends the call with
+ * ALP_ERR_CUDA.  It must not call back into the context.  An input that is
+ * rejected may get no call.  fn NULL: outputs are owned by the context again. */
+enum { ALP_ALLOC_OFF = 5, ALP_ALLOC_VALID = 6, ALP_ALLOC_PTRS = 7 };
+typedef int (*alp_alloc_fn)(void* user, int64_t n, void** ptrs);
+int alp_set_output_alloc(alp_ctx* ctx, alp_alloc_fn fn, void* user);
+
 /* lex_int: bytes -> tokens (futhark/lexer.fut:174-178 through
  * src/Alpacc/Generator/Futhark/Generator.hs:70-75). */
 int alp_lex(alp_ctx* ctx, const uint8_t* d_in, int64_t n, uint32_t** d_term, int64_t** d_start,
