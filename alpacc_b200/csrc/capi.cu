@@ -21,6 +21,7 @@
 #include "lexer.cuh"
 #include "lex3.cuh"
 #include "parser.cuh"
+#include "tree.cuh"
 #include "mlp.cuh"
 #include "spec.cuh"
 #include "spec3.cuh"
@@ -89,11 +90,13 @@ struct alp_ctx {
     bool has_parser = false;
     ParseTables pt{};
     ParseHost ph{};
+    bool tree = false;                    // the grammar fits parse_tree_kernel's compact tables
+    TreeTables tt{};
     // ---- memory ----
     std::vector<void*> owned;             // table allocations
     DevBuf scratch;                       // look-back status words, results
     DevBuf out[8];                        // context-owned outputs
-    DevBuf tmp[32];                       // intermediates
+    DevBuf tmp[40];                       // intermediates
     long long* h_stage = nullptr;         // pinned staging for small host->device values
     // alp_parse_host's host buffers: the node fields the searches leave alone start to
     // the host as soon as the expansion has written them
@@ -518,8 +521,10 @@ enum {
     T_HIN = 0, T_TTERM, T_TSTART, T_TEND, T_PID, T_TSUMS, T_VBUF, T_BRBUF, T_DSBUF,
     T_N_TMIN, T_N_M32, T_N_M1024, T_N_SVAL, T_N_SIDX, T_N_SLEN, T_N_ESC,
     T_B_TMIN, T_B_M32, T_B_M1024, T_B_SVAL, T_B_SIDX, T_B_SLEN, T_B_ESC,
-    T_DOCOFF, T_TOKOFF, T_NODEOFF, T_BROFF, T_DVALID, T_NARROW, T_HOFF, T_CNT
+    T_DOCOFF, T_TOKOFF, T_NODEOFF, T_BROFF, T_DVALID, T_NARROW, T_HOFF,
+    T_TR_TILES, T_TR_ESC, T_TR_STAIR, T_CNT
 };
+static_assert(T_CNT <= 40, "alp_ctx::tmp");
 
 struct ParseOut {
     int64_t* parent;
@@ -528,6 +533,8 @@ struct ParseOut {
     int64_t* start;
     int64_t* end;
 };
+
+int load_tree(alp_ctx* ctx);
 
 int set_result(alp_ctx* ctx, AlpResult* d_res, int valid) {
     memset(ctx->h_res, 0, sizeof(AlpResult));
@@ -1011,8 +1018,10 @@ int put_doc_off(alp_ctx* ctx, long long n) {
 // documents land in tmp[T_NODEOFF].
 // Output buffers for N nodes (context-owned when ctx_out) and the node and
 // bracket intermediates for N nodes and K kept brackets.
-// `exact`: N is the node count, for which a caller's allocator can be asked.
-int parse_buffers(alp_ctx* ctx, ParseOut* o, int ctx_out, long long N, long long K, ParseArgs& a, bool exact = true) {
+// `exact`: N is the node count, for which a caller's allocator can be asked.  `general`:
+// with the node values and brackets of the general kernels.
+int parse_buffers(alp_ctx* ctx, ParseOut* o, int ctx_out, long long N, long long K, ParseArgs& a, bool exact = true,
+                  bool general = true) {
     int rc;
     if (ctx_out && ctx->alloc_fn && exact) {
         void* p[5] = {};
@@ -1033,8 +1042,8 @@ int parse_buffers(alp_ctx* ctx, ParseOut* o, int ctx_out, long long N, long long
         o->start = (int64_t*)ctx->out[6].p;
         o->end = (int64_t*)ctx->out[7].p;
     }
-    if ((rc = grow(ctx, ctx->tmp[T_VBUF], N * 4 + 8)) || (rc = grow(ctx, ctx->tmp[T_BRBUF], K * 4 + 8)) ||
-        (rc = grow(ctx, ctx->tmp[T_DSBUF], K * 4 + 8)))
+    if (general && ((rc = grow(ctx, ctx->tmp[T_VBUF], N * 4 + 8)) || (rc = grow(ctx, ctx->tmp[T_BRBUF], K * 4 + 8)) ||
+                    (rc = grow(ctx, ctx->tmp[T_DSBUF], K * 4 + 8))))
         return rc;
     a.tag = o->tag;
     a.kind = o->kind;
@@ -1059,13 +1068,12 @@ inline const void* fused_expand_for(int q, int k) {
     return (const void*)parse_expand_kernel<0, 0, true>;
 }
 
-// Dynamic shared memory of an expand launch (*sm): its tables, position records and
-// node owners, and past them up to EX_SPAN_BYTES more for the tile's token spans, as
+// Dynamic shared memory of an expand or tree launch (*sm): `base` for its tables,
+// positions and node owners, and past them up to EX_SPAN_BYTES more for the tile's token spans, as
 // many as leave room for the CTAs per SM that run without them (or the tuned count).
-int expand_smem(alp_ctx* ctx, const void* fn, ParseArgs& a, size_t* sm) {
-    const size_t base = expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack);
+int expand_smem(alp_ctx* ctx, const void* fn, size_t base, int* span_cap, size_t* sm) {
     *sm = base;
-    a.span_cap = 0;
+    *span_cap = 0;
     int fit = 0, per_sm = 0, reserved = 0, optin = 0;
     cudaFuncAttributes fa;
     CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)base));
@@ -1083,7 +1091,7 @@ int expand_smem(alp_ctx* ctx, const void* fn, ParseArgs& a, size_t* sm) {
     CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(base + room)));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit2, fn, PP_THREADS, base + room));
     if (fit2 < ctas) return ALP_OK;  // token spans through L1, as without the stage
-    a.span_cap = (int)(room / 8);     // a multiple of 4
+    *span_cap = (int)(room / 8);      // a multiple of 4
     *sm = base + (size_t)room;
     return ALP_OK;
 }
@@ -1095,6 +1103,84 @@ int expand_grid(alp_ctx* ctx, const void* fn, size_t sm2, long long tiles, unsig
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, fn, PP_THREADS, sm2));
     const long long x = (long long)persistent_ctas(per2, ctx->tune.expand_ctas) * sms;
     *g = (unsigned)(x < tiles ? x : tiles);
+    return ALP_OK;
+}
+
+// parse_tree_kernel and the searches that leave a tile, for the positions, pair ids and
+// scanned tile sums of `a`.  parent null: no parents.  With a.dL the counts are in device
+// memory, a.L and a.cap_nodes capacities.
+TreeArgs tree_args(alp_ctx* ctx, const ParseArgs& a, long long* parent) {
+    TreeArgs t;
+    memset(&t, 0, sizeof t);
+    t.t = ctx->tt;
+    t.sent_l = ctx->pt.start;
+    t.sent_r = ctx->pt.end;
+    t.P = a.P;
+    t.pid = a.pid;
+    t.pstart = a.pstart;
+    t.pend = a.pend;
+    t.L = a.L;
+    t.n_docs = a.n_docs;
+    t.dL = a.dL;
+    t.tile_sums = a.tile_sums;
+    t.tok_off = (const long long*)ctx->tmp[T_TOKOFF].p;
+    t.tag = a.tag;
+    t.kind = a.kind;
+    t.nstart = a.nstart;
+    t.nend = a.nend;
+    t.parent = parent;
+    t.node_off = a.node_off;
+    t.doc_valid = a.doc_valid;
+    if (!a.subst_terminals) t.t.rec = t.t.plain;
+    t.cap_nodes = a.cap_nodes;
+    return t;
+}
+
+int tree_buffers(alp_ctx* ctx, TreeArgs& t) {
+    const long long tiles = (t.L + PP_TILE - 1) / PP_TILE, n32 = (tiles + 31) / 32, n1024 = (tiles + 1023) / 1024;
+    int rc;
+    if ((rc = grow(ctx, ctx->tmp[T_TR_TILES], (size_t)tiles * (sizeof(TreeTile) + 4) + 4 * (size_t)(n32 + n1024))) ||
+        (rc = grow(ctx, ctx->tmp[T_TR_ESC], (size_t)(t.cap_nodes + tiles) * 8)) ||
+        (rc = grow(ctx, ctx->tmp[T_TR_STAIR], (size_t)tiles * PP_TILE * 8)))
+        return rc;
+    t.tiles = (TreeTile*)ctx->tmp[T_TR_TILES].p;
+    t.tile_min = (int32_t*)(t.tiles + tiles);
+    t.m32 = t.tile_min + tiles;
+    t.m1024 = t.m32 + n32;
+    t.esc = (uint2*)ctx->tmp[T_TR_ESC].p;
+    t.esc_cap = t.cap_nodes + tiles;
+    t.stair = (uint2*)ctx->tmp[T_TR_STAIR].p;
+    return ALP_OK;
+}
+
+int run_tree(alp_ctx* ctx, TreeArgs& t, bool one) {
+    const long long tiles = (t.L + PP_TILE - 1) / PP_TILE;
+    int rc;
+    const void* fn = one ? (const void*)parse_tree_kernel<true> : (const void*)parse_tree_kernel<false>;
+    size_t sm = 0;
+    unsigned g = 1;
+    if ((rc = tree_buffers(ctx, t)) ||
+        (rc = expand_smem(ctx, fn, tree_smem_bytes(ctx->tt.n_pairs, ctx->tt.n_pseq, ctx->tt.n_stack, one), &t.span_cap, &sm)) ||
+        (rc = expand_grid(ctx, fn, sm, tiles, &g)))
+        return rc;
+    mark(ctx, "start");
+    {
+        void* args[] = {&t};
+        CK(cudaLaunchKernel(fn, dim3(g), dim3(PP_THREADS), args, sm, ctx->stream));
+    }
+    mark(ctx, "parse_tree_kernel");
+    return ALP_OK;
+}
+
+int run_tree_escapes(alp_ctx* ctx, TreeArgs& t) {
+    const long long tiles = (t.L + PP_TILE - 1) / PP_TILE;
+    mark(ctx, "start");
+    tree_levels_kernel<<<(unsigned)(((tiles + 31) / 32 + 255) / 256), 256, 0, ctx->stream>>>(t, tiles);
+    CK(cudaGetLastError());
+    const long long g = (tiles + 7) / 8;
+    tree_escape_kernel<<<(unsigned)(g < 148 * 8 ? g : 148 * 8), 256, 0, ctx->stream>>>(t, tiles);
+    CK(cudaGetLastError());
+    mark(ctx, "tree_levels+tree_escape");
     return ALP_OK;
 }
 
@@ -1139,6 +1225,7 @@ int parse_positions(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, Pa
         return fail(ctx, ALP_ERR_TABLE, "parser tables too large for shared memory");
     size_t sm2 = expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack);
     long long N = 0, B = 0, K = 0;
+    TreeArgs tree;
     const bool fits32 = (unsigned long long)L * (unsigned long long)(ctx->ph.max_prods + 1) < (1ull << 32) &&
                         (unsigned long long)L * (unsigned long long)(ctx->ph.max_brackets + 1) < (1ull << 32);
     const bool fused = !ctx->tune.parse_split && fits32 && ctx->est_nodes > 0;
@@ -1224,17 +1311,23 @@ int parse_positions(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, Pa
             *n_node = N;
             return fail(ctx, ALP_ERR_CAPACITY, "node buffer too small (%lld needed)", (long long)N);
         }
-        if ((rc = parse_buffers(ctx, o, ctx_out, N, K, a))) return rc;
-        // one document: the expansion's thread-level sums need no restarts
-        const void* ex = nd == 1 ? (const void*)parse_expand_kernel<0, 0, false, true>
-                                 : (const void*)parse_expand_kernel<0, 0, false, false>;
-        if ((rc = expand_smem(ctx, ex, a, &sm2)) || (rc = expand_grid(ctx, ex, sm2, tiles, &g_expand))) return rc;
-        mark(ctx, "start");
-        {
-            void* args[] = {&a};
-            CK(cudaLaunchKernel(ex, dim3(g_expand), dim3(PP_THREADS), args, sm2, ctx->stream));
+        if ((rc = parse_buffers(ctx, o, ctx_out, N, K, a, true, !ctx->tree))) return rc;
+        if (ctx->tree) {
+            tree = tree_args(ctx, a, want_tree ? (long long*)o->parent : nullptr);
+            if ((rc = run_tree(ctx, tree, nd == 1))) return rc;
+        } else {
+            const void* ex = (const void*)parse_expand_kernel<0, 0, false>;
+            if ((rc = expand_smem(ctx, ex, expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack),
+                                  &a.span_cap, &sm2)) ||
+                (rc = expand_grid(ctx, ex, sm2, tiles, &g_expand)))
+                return rc;
+            mark(ctx, "start");
+            {
+                void* args[] = {&a};
+                CK(cudaLaunchKernel(ex, dim3(g_expand), dim3(PP_THREADS), args, sm2, ctx->stream));
+            }
+            mark(ctx, "parse_expand_kernel");
         }
-        mark(ctx, "parse_expand_kernel");
     }
     ctx->last_positions = L;
     ctx->last_brackets = B;
@@ -1264,7 +1357,9 @@ int parse_positions(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, Pa
             CK(cudaMemcpyAsync(h.end, o->end, (size_t)N * 8, cudaMemcpyDeviceToHost, ctx->cp_out));
         }
     }
-    if (want_tree && !ctx->prof) {
+    if (ctx->tree && !fused) {
+        if ((rc = run_tree_escapes(ctx, tree))) return rc;
+    } else if (want_tree && !ctx->prof) {
         // the node and bracket searches share nothing but the result block (atomic
         // error bits) and document validity (cleared only): the bracket search runs on a
         // second stream beside the node search, each half-filling the SMs alone
@@ -1469,6 +1564,30 @@ inline unsigned grid_for(long long n) {
     return (unsigned)(g < 1 ? 1 : g);
 }
 
+// The compact tables of parse_tree_kernel, where the grammar fits them.
+int load_tree(alp_ctx* ctx) {
+    TreeHost h;
+    if (!build_tree_tables(ctx->ph.pairs, ctx->ph.pair_use, ctx->ph.stack, ctx->ph.pseq, ctx->ph.arity, ctx->ph.pterm, h))
+        return ALP_OK;
+    TreeTables& t = ctx->tt;
+    t.n_pairs = (int)ctx->ph.pairs.size();
+    t.n_pseq = (int)ctx->ph.pseq.size();
+    t.n_stack = (int)ctx->ph.stack.size();
+    if (tree_smem_bytes(t.n_pairs, t.n_pseq, t.n_stack, false) > 220 * 1024) return ALP_OK;
+    const uint32_t *pairs, *rec, *plain;
+    int rc;
+    if ((rc = upload(ctx, h.pairs.data(), h.pairs.size(), &pairs)) ||
+        (rc = upload(ctx, h.rec.data(), h.rec.size(), &rec)) ||
+        (rc = upload(ctx, h.plain.data(), h.plain.size(), &plain)) ||
+        (rc = upload(ctx, h.stack.data(), h.stack.size(), &t.stack)))
+        return rc;
+    t.pairs = reinterpret_cast<const uint2*>(pairs);
+    t.rec = reinterpret_cast<const uint2*>(rec);
+    t.plain = reinterpret_cast<const uint2*>(plain);
+    ctx->tree = true;
+    return ALP_OK;
+}
+
 // The tail of alp_parse_host and alp_parse_batch_host: after the parse (rc) the
 // tree's N nodes to the caller's host arrays (capacity cap), with parents and
 // spans as 32-bit values widened on the host when parse_positions narrowed the
@@ -1572,6 +1691,7 @@ int alp_ctx_create(const void* blob, size_t len, int device, alp_ctx** out) {
     if (!rc && hl) rc = load_lexer(ctx, r);
     if (!rc && hp) rc = load_parser(ctx->pt, ctx->ph, r.p, r.e, ctx->owned, ctx->err);
     if (!rc && hp) ctx->has_parser = true;
+    if (!rc && hp) rc = load_tree(ctx);
     if (!rc && hl && hp) {
         // the parser indexes its key table with the lexer's terminal ids
         const uint32_t T = (uint32_t)ctx->pt.T;
@@ -3691,9 +3811,9 @@ int parse_positions_dev(alp_ctx* ctx, long long Lcap, const long long* dL, long 
     if ((rc = grow(ctx, ctx->tmp[T_PID], (size_t)Lcap * 2 + 64)) ||
         (rc = grow(ctx, ctx->tmp[T_TSUMS], (tiles + tiles / ST_CHUNK + 2) * sizeof(PosSums))) ||
         (rc = grow(ctx, ctx->tmp[T_BROFF], (size_t)(nd + 1) * 8)) || (rc = grow(ctx, ctx->scratch, 256)) ||
-        (rc = grow(ctx, ctx->tmp[T_VBUF], (size_t)cap_nodes * 4 + 8)) ||
-        (rc = grow(ctx, ctx->tmp[T_BRBUF], (size_t)cap_brs * 4 + 8)) ||
-        (rc = grow(ctx, ctx->tmp[T_DSBUF], (size_t)cap_brs * 4 + 8)))
+        (!ctx->tree && ((rc = grow(ctx, ctx->tmp[T_VBUF], (size_t)cap_nodes * 4 + 8)) ||
+                        (rc = grow(ctx, ctx->tmp[T_BRBUF], (size_t)cap_brs * 4 + 8)) ||
+                        (rc = grow(ctx, ctx->tmp[T_DSBUF], (size_t)cap_brs * 4 + 8)))))
         return rc;
     AlpResult* d_res = reinterpret_cast<AlpResult*>(ctx->scratch.p);
     ParseArgs a;
@@ -3727,7 +3847,9 @@ int parse_positions_dev(alp_ctx* ctx, long long Lcap, const long long* dL, long 
     if (expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack) > 220 * 1024)
         return fail(ctx, ALP_ERR_TABLE, "parser tables too large for shared memory");
     size_t sm2 = 0;
-    if ((rc = expand_smem(ctx, (const void*)parse_expand_kernel<0, 0, false>, a, &sm2))) return rc;
+    if ((rc = expand_smem(ctx, (const void*)parse_expand_kernel<0, 0, false>,
+                          expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack), &a.span_cap, &sm2)))
+        return rc;
     CK(cudaFuncSetAttribute(pairs_kernel_for(ctx->pt.q, ctx->pt.k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, pairs_kernel_for(ctx->pt.q, ctx->pt.k), PP_THREADS, sm1));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, parse_expand_kernel<0, 0, false>, PP_THREADS, sm2));
@@ -3746,6 +3868,11 @@ int parse_positions_dev(alp_ctx* ctx, long long Lcap, const long long* dL, long 
         scan_tiles_kernel<<<(unsigned)chunks, ST_CHUNK, 0, ctx->stream>>>(a.tile_sums, tiles, csum, d_res, a.node_off,
                                                                          a.br_off, nd, dL);
         CK(cudaGetLastError());
+    }
+    if (ctx->tree) {
+        TreeArgs t = tree_args(ctx, a, (long long*)o.parent);
+        if ((rc = run_tree(ctx, t, false))) return rc;
+        return run_tree_escapes(ctx, t);
     }
     parse_expand_kernel<0, 0, false><<<(unsigned)(x2 < tiles ? x2 : tiles), PP_THREADS, sm2, ctx->stream>>>(a);
     CK(cudaGetLastError());
@@ -3820,6 +3947,8 @@ alp_ctx* child_ctx(const alp_ctx* p) {
     c->has_parser = p->has_parser;
     c->pt = p->pt;
     c->ph = p->ph;
+    c->tree = p->tree;
+    c->tt = p->tt;
     c->tune = p->tune;
     return c;
 }

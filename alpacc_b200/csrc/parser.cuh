@@ -4,6 +4,8 @@
 //   K1 parse_pairs   -- keys over ⊢ tokens ⊣ (get_key, lines 117-122), the pair
 //                       lookup (lines 130-148) and one decoupled look-back scan
 //                       of every per-position count the later passes need;
+// (K2 to K4 are the general form: shards of a document, the fused position pass and
+// grammars outside the compact tables; else parse_tree_kernel does all three, tree.cuh.)
 //   K2 parse_expand  -- the segmented copies of stacks and productions
 //                       (lines 216-233), node tags, terminal-node spans
 //                       (lines 305-329), the value sequences of the two
@@ -59,6 +61,10 @@ struct ParseHost {
     // host copies for the pairs at shard boundaries (alp_parse_shard_*)
     std::vector<uint16_t> key_index;
     std::vector<PairInfo> pairs;
+    // and for the compact tables of parse_tree_kernel
+    std::vector<uint32_t> stack, pseq;
+    std::vector<int32_t> arity, pterm;
+    std::vector<uint8_t> pair_use;  // 1: at positions other than ⊢, 2: at ⊢
     uint32_t T = 0, empty = 0, start = 0, end = 0;
 };
 
@@ -109,6 +115,7 @@ inline int load_parser(ParseTables& pt, ParseHost& ph, const uint8_t* p, const u
         if (space > (1ll << 24)) { err = "key space too large for the direct key index"; return 4; }
     }
     std::vector<uint16_t> index((size_t)space, 0xffff);
+    ph.pair_use.assign(n_pairs, 0);
     for (uint32_t i = 0; i < n_keys; ++i) {
         long long x = 0;
         for (uint32_t j = 0; j < W; ++j) {
@@ -118,6 +125,7 @@ inline int load_parser(ParseTables& pt, ParseHost& ph, const uint8_t* p, const u
         }
         if (key_pair[i] >= n_pairs) { err = "key names a pair out of range"; return 4; }
         index[(size_t)x] = (uint16_t)key_pair[i];
+        ph.pair_use[key_pair[i]] |= keys[(size_t)i * W + q] == start ? 2 : 1;
     }
     std::vector<PairInfo> info(n_pairs);
     int maxp = 0, maxb = 0;
@@ -203,6 +211,10 @@ inline int load_parser(ParseTables& pt, ParseHost& ph, const uint8_t* p, const u
     ph.max_prods = maxp; ph.max_brackets = maxb; ph.key_space = space;
     ph.key_index = std::move(index);
     ph.pairs = info;
+    ph.stack = std::move(stack);
+    ph.pseq = std::move(pseq);
+    ph.arity = std::move(arity);
+    ph.pterm = std::move(pterm);
     ph.T = T; ph.empty = empty; ph.start = start; ph.end = end;
     return 0;
 }
@@ -236,10 +248,12 @@ struct __align__(16) PosSums {
     uint32_t heads;   // ⊢ positions
     int32_t hpos;     // position of the last ⊢ (-1: none)
     uint32_t cls;     // bracket pairs closed between a position and the one before it
+    uint32_t dnodes;  // productions since the last ⊢
 };
 
 __device__ __forceinline__ void possums_zero(PosSums& s) {
     s.nodes = 0; s.brs = 0; s.depth = 0; s.v = 0; s.terms = 0; s.heads = 0; s.hpos = -1; s.cls = 0;
+    s.dnodes = 0;
 }
 __device__ __forceinline__ PosSums ps_combine(const PosSums& a, const PosSums& b) {
     PosSums r;
@@ -252,53 +266,7 @@ __device__ __forceinline__ PosSums ps_combine(const PosSums& a, const PosSums& b
     r.terms = h ? b.terms : a.terms + b.terms;
     r.hpos = h ? b.hpos : a.hpos;
     r.cls = a.cls + b.cls;
-    return r;
-}
-// ps_combine where all positions belong to one document: its only ⊢ is position 0,
-// before which every sum is zero, so that restarting there is the same as adding.
-// The ⊢ count and position are then not needed (left 0).
-template <bool ONE>
-__device__ __forceinline__ PosSums ps_join(const PosSums& a, const PosSums& b) {
-    if (!ONE) return ps_combine(a, b);
-    PosSums r;
-    r.nodes = a.nodes + b.nodes;
-    r.brs = a.brs + b.brs;
-    r.heads = 0;
-    r.depth = a.depth + b.depth;
-    r.v = a.v + b.v;
-    r.terms = a.terms + b.terms;
-    r.hpos = 0;
-    r.cls = a.cls + b.cls;
-    return r;
-}
-// The one-document forms of the warp scan and shift: no ⊢ anywhere but position 0
-// (whose sums before it are zero), so the six counted fields are plain prefix sums
-// and the ⊢ fields stay 0.
-__device__ __forceinline__ PosSums ps_warp_scan_one(PosSums x, int lane) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t on = __shfl_up_sync(ALP_FULL_MASK, x.nodes, d);
-        const uint32_t ob = __shfl_up_sync(ALP_FULL_MASK, x.brs, d);
-        const int32_t od = __shfl_up_sync(ALP_FULL_MASK, x.depth, d);
-        const int32_t ov = __shfl_up_sync(ALP_FULL_MASK, x.v, d);
-        const uint32_t ot = __shfl_up_sync(ALP_FULL_MASK, x.terms, d);
-        const uint32_t oc = __shfl_up_sync(ALP_FULL_MASK, x.cls, d);
-        if (lane >= d) { x.nodes += on; x.brs += ob; x.depth += od; x.v += ov; x.terms += ot; x.cls += oc; }
-    }
-    x.heads = 0;
-    x.hpos = 0;
-    return x;
-}
-__device__ __forceinline__ PosSums ps_shfl_up_one(const PosSums& x, int d) {
-    PosSums r;
-    r.nodes = __shfl_up_sync(ALP_FULL_MASK, x.nodes, d);
-    r.brs = __shfl_up_sync(ALP_FULL_MASK, x.brs, d);
-    r.depth = __shfl_up_sync(ALP_FULL_MASK, x.depth, d);
-    r.v = __shfl_up_sync(ALP_FULL_MASK, x.v, d);
-    r.terms = __shfl_up_sync(ALP_FULL_MASK, x.terms, d);
-    r.cls = __shfl_up_sync(ALP_FULL_MASK, x.cls, d);
-    r.heads = 0;
-    r.hpos = 0;
+    r.dnodes = h ? b.dnodes : a.dnodes + b.dnodes;
     return r;
 }
 __device__ __forceinline__ PosSums ps_shfl_up(const PosSums& x, int d) {
@@ -311,6 +279,7 @@ __device__ __forceinline__ PosSums ps_shfl_up(const PosSums& x, int d) {
     r.heads = __shfl_up_sync(ALP_FULL_MASK, x.heads, d);
     r.hpos = __shfl_up_sync(ALP_FULL_MASK, x.hpos, d);
     r.cls = __shfl_up_sync(ALP_FULL_MASK, x.cls, d);
+    r.dnodes = __shfl_up_sync(ALP_FULL_MASK, x.dnodes, d);
     return r;
 }
 // inclusive warp scan (lanes in order); a warp without a ⊢ needs plain sums
@@ -326,6 +295,7 @@ __device__ __forceinline__ PosSums ps_warp_scan(PosSums x, int lane) {
             const uint32_t oc = __shfl_up_sync(ALP_FULL_MASK, x.cls, d);
             if (lane >= d) { x.nodes += on; x.brs += ob; x.depth += od; x.v += ov; x.terms += ot; x.cls += oc; }
         }
+        x.dnodes = x.nodes;  // no ⊢: the same counts
         return x;
     }
 #pragma unroll
@@ -335,17 +305,6 @@ __device__ __forceinline__ PosSums ps_warp_scan(PosSums x, int lane) {
     }
     return x;
 }
-__device__ __forceinline__ PosSums ps_elem(const PairInfo* s_pi, uint16_t p, bool head, long long i) {
-    PosSums e;
-    possums_zero(e);
-    if (p != NO_PAIR) {
-        const PairInfo& pi = s_pi[p];
-        e.nodes = pi.n_prod; e.brs = pi.n_br; e.depth = pi.d_depth; e.v = pi.d_v; e.terms = pi.n_term;
-    }
-    if (head) { e.heads = 1; e.hpos = (int32_t)i; }
-    return e;
-}
-
 // Brackets closed between adjacent positions: a pair's brackets are its
 // rights, then its lefts, so position p's first rights close position p-1's
 // top lefts, min(lefts of p-1, rights of p) of them, unless p starts a
@@ -533,7 +492,7 @@ __global__ void __launch_bounds__(PP_THREADS, 3) parse_pairs_kernel(ParseArgs a)
                 uint32_t nl = 0;
                 if (ids[j] != NO_PAIR) {
                     const PairInfo& pi = s_pi[ids[j]];
-                    e.nodes = pi.n_prod; e.brs = pi.n_br; e.depth = pi.d_depth; e.v = pi.d_v; e.terms = pi.n_term;
+                    e.nodes = pi.n_prod; e.dnodes = pi.n_prod; e.brs = pi.n_br; e.depth = pi.d_depth; e.v = pi.d_v; e.terms = pi.n_term;
                     nl = pair_lefts(pi);
                     if (!head && pv) e.cls = min(lprev, (uint32_t)pi.n_br - nl);  // adj_closed
                 }
@@ -567,6 +526,7 @@ __global__ void __launch_bounds__(PP_THREADS, 3) parse_pairs_kernel(ParseArgs a)
         inc.cls = __reduce_add_sync(ALP_FULL_MASK, acc.cls);
         inc.heads = 0;
         inc.hpos = -1;
+        inc.dnodes = inc.nodes;
     } else {
         inc = ps_warp_scan(acc, lane);
     }
@@ -646,6 +606,7 @@ __global__ void __launch_bounds__(ST_CHUNK) scan_tiles_kernel(PosSums* s, long l
             last.heads = __shfl_sync(ALP_FULL_MASK, inc.heads, 31);
             last.hpos = __shfl_sync(ALP_FULL_MASK, inc.hpos, 31);
             last.cls = __shfl_sync(ALP_FULL_MASK, inc.cls, 31);
+            last.dnodes = __shfl_sync(ALP_FULL_MASK, inc.dnodes, 31);
             carry = ps_combine(carry, last);
         }
         if (lane == 0) s_carry = carry;
@@ -758,21 +719,19 @@ __host__ __device__ inline size_t expand_smem_bytes(int n_pairs, int n_pseq, int
     return expand_tables_bytes(n_pairs, n_pseq, n_stack) + EX_POS_BYTES + 2 * (size_t)EX_WIN;
 }
 
-// Pair ids and (TERMS) terminals of the PP_ITEMS positions from i0 as two
-// 8-byte words (one vector load each when all are in range; ids past the end
-// read as no pair).
-template <bool TERMS>
+// Pair ids and terminals of the PP_ITEMS positions from i0 as two 8-byte words
+// (one vector load each when all are in range; ids past the end read as no pair).
 __device__ __forceinline__ void ex_words(const ParseArgs& a, long long i0, uint2& w, uint2& t) {
     static_assert(PP_ITEMS == 4, "a thread's positions are one 8-byte word");
     if (i0 + PP_ITEMS <= a.L) {
         w = __ldg(reinterpret_cast<const uint2*>(a.pid + i0));
-        if (TERMS) t = __ldg(reinterpret_cast<const uint2*>(a.P + i0));
+        t = __ldg(reinterpret_cast<const uint2*>(a.P + i0));
     } else {
         uint32_t x[PP_ITEMS], y[PP_ITEMS];
 #pragma unroll
         for (int j = 0; j < PP_ITEMS; ++j) {
             x[j] = i0 + j < a.L ? a.pid[i0 + j] : NO_PAIR;
-            y[j] = (TERMS && i0 + j < a.L) ? a.P[i0 + j] : 0xffffu;
+            y[j] = i0 + j < a.L ? a.P[i0 + j] : 0xffffu;
         }
         w = make_uint2(x[0] | (x[1] << 16), x[2] | (x[3] << 16));
         t = make_uint2(y[0] | (y[1] << 16), y[2] | (y[3] << 16));
@@ -790,12 +749,14 @@ __device__ __forceinline__ PosSums ps_ld(const PosSums* p) {
     PosSums r;
     r.nodes = x.x; r.brs = x.y; r.depth = (int32_t)x.z; r.v = (int32_t)x.w;
     r.terms = y.x; r.heads = y.y; r.hpos = (int32_t)y.z; r.cls = y.w;
+    r.dnodes = v[2].x;
     return r;
 }
 __device__ __forceinline__ void ps_st(PosSums* p, const PosSums& r) {
     volatile uint4* v = reinterpret_cast<volatile uint4*>(p);
     v[0].x = r.nodes; v[0].y = r.brs; v[0].z = (uint32_t)r.depth; v[0].w = (uint32_t)r.v;
     v[1].x = r.terms; v[1].y = r.heads; v[1].z = (uint32_t)r.hpos; v[1].w = r.cls;
+    v[2].x = r.dnodes;
 }
 __device__ __forceinline__ PosSums ps_shfl_down(const PosSums& x, int d) {
     PosSums r;
@@ -807,6 +768,7 @@ __device__ __forceinline__ PosSums ps_shfl_down(const PosSums& x, int d) {
     r.heads = __shfl_down_sync(ALP_FULL_MASK, x.heads, d);
     r.hpos = __shfl_down_sync(ALP_FULL_MASK, x.hpos, d);
     r.cls = __shfl_down_sync(ALP_FULL_MASK, x.cls, d);
+    r.dnodes = __shfl_down_sync(ALP_FULL_MASK, x.dnodes, d);
     return r;
 }
 __device__ __forceinline__ PosSums ps_lookback(const ParseArgs& a, long long tile, const PosSums& agg) {
@@ -851,6 +813,7 @@ __device__ __forceinline__ PosSums ps_lookback(const ParseArgs& a, long long til
         win.heads = __shfl_sync(ALP_FULL_MASK, x.heads, 0);
         win.hpos = __shfl_sync(ALP_FULL_MASK, x.hpos, 0);
         win.cls = __shfl_sync(ALP_FULL_MASK, x.cls, 0);
+        win.dnodes = __shfl_sync(ALP_FULL_MASK, x.dnodes, 0);
         acc = ps_combine(win, acc);
         if (pm) break;
         end -= 32;
@@ -868,9 +831,7 @@ __device__ __forceinline__ PosSums ps_lookback(const ParseArgs& a, long long til
 // exclusive position sums from a look-back over earlier tiles (tiles taken in
 // ticket order, so every tile a look-back waits for is running or done).  The
 // pair kernel, the tile-sum scans and the pair-id array are then not needed.
-// ONE: the positions are one document (not a shard of one): the thread-level
-// sums are plain sums and every position's document is document 0.
-template <int QT, int KT, bool FUSED, bool ONE = false>
+template <int QT, int KT, bool FUSED>
 __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     PairInfo* s_pi = reinterpret_cast<PairInfo*>(smem);
@@ -905,7 +866,7 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a
     // (not fused) this thread's pair ids and terminals, one tile ahead (loads in
     // flight while the block works on the current tile)
     uint2 nw = make_uint2(0, 0), nt = make_uint2(0, 0);
-    if (!FUSED) ex_words<!ONE>(a, (long long)blockIdx.x * PP_TILE + tid * PP_ITEMS, nw, nt);
+    if (!FUSED) ex_words(a, (long long)blockIdx.x * PP_TILE + tid * PP_ITEMS, nw, nt);
     for (long long it = blockIdx.x;; it += gridDim.x) {
         __syncthreads();  // the previous tile is done with the shared arrays
         long long tile = it;
@@ -966,26 +927,20 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a
         } else {
             tp = a.shard ? ps_combine(a.pre, a.tile_sums[tile]) : a.tile_sums[tile];
             ids[0] = (uint16_t)nw.x; ids[1] = (uint16_t)(nw.x >> 16); ids[2] = (uint16_t)nw.y; ids[3] = (uint16_t)(nw.y >> 16);
-            if (ONE) {
-                // one document: its ⊢ is position 0 and its ⊣ position L - 1
-                if (i0 == 0) hm = 1u;
-                if (a.L - 1 >= i0 && a.L - 1 < i0 + PP_ITEMS) em = 1u << (uint32_t)(a.L - 1 - i0);
-            } else {
-                const uint32_t c[PP_ITEMS] = {nt.x & 0xffffu, nt.x >> 16, nt.y & 0xffffu, nt.y >> 16};
+            const uint32_t c[PP_ITEMS] = {nt.x & 0xffffu, nt.x >> 16, nt.y & 0xffffu, nt.y >> 16};
 #pragma unroll
-                for (int j = 0; j < PP_ITEMS; ++j) {
-                    if (i0 + j < a.L) {
-                        if (c[j] == SL) hm |= 1u << j;
-                        if (c[j] == SR) em |= 1u << j;
-                    }
+            for (int j = 0; j < PP_ITEMS; ++j) {
+                if (i0 + j < a.L) {
+                    if (c[j] == SL) hm |= 1u << j;
+                    if (c[j] == SR) em |= 1u << j;
                 }
             }
-            if (tile + gridDim.x < n_tiles) ex_words<!ONE>(a, i0 + (long long)gridDim.x * PP_TILE, nw, nt);
+            if (tile + gridDim.x < n_tiles) ex_words(a, i0 + (long long)gridDim.x * PP_TILE, nw, nt);
             if (lane == 0 && i0 > 0 && i0 - 1 < a.L) prev_id = a.pid[i0 - 1];
             else if (lane == 0 && i0 == 0 && a.shard) prev_id = a.prev_pair;
             if (lane == 31 && i0 + PP_ITEMS < a.L) {
                 next_id = a.pid[i0 + PP_ITEMS];
-                next_head = !ONE && (uint32_t)a.P[i0 + PP_ITEMS] == SL;  // one document: no ⊢ after position 0
+                next_head = (uint32_t)a.P[i0 + PP_ITEMS] == SL;
             } else if (lane == 31 && i0 + PP_ITEMS == a.L && a.shard) {
                 next_id = a.next_pair;  // the next shard's first position (never a document head)
             }
@@ -1012,13 +967,13 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a
                     uint32_t nl = 0;
                     if (ids[j] != NO_PAIR) {
                         const PairInfo& pi = s_pi[ids[j]];
-                        e.nodes = pi.n_prod; e.brs = pi.n_br; e.depth = pi.d_depth; e.v = pi.d_v; e.terms = pi.n_term;
+                        e.nodes = pi.n_prod; e.dnodes = pi.n_prod; e.brs = pi.n_br; e.depth = pi.d_depth; e.v = pi.d_v; e.terms = pi.n_term;
                         nl = pair_lefts(pi);
                         if (!head && pv) e.cls = min(lprev, (uint32_t)pi.n_br - nl);
                     }
-                    if (head && !ONE) { e.heads = 1; e.hpos = (int32_t)(i0 + j); }
+                    if (head) { e.heads = 1; e.hpos = (int32_t)(i0 + j); }
                     cl[j] = e.cls;
-                    mine = ps_join<ONE>(mine, e);
+                    mine = ps_combine(mine, e);
                     lprev = nl;
                     pv = ids[j] != NO_PAIR;
                 } else if (a.shard && i0 + j == a.L && pv && a.next_pair != NO_PAIR) {
@@ -1034,16 +989,16 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a
                                    ? adj_closed(s_pi, ids[PP_ITEMS - 1], next_id, next_head) : 0u;
             }
         }
-        const PosSums inc = ONE ? ps_warp_scan_one(mine, lane) : ps_warp_scan(mine, lane);
-        PosSums ex = ONE ? ps_shfl_up_one(inc, 1) : ps_shfl_up(inc, 1);
+        const PosSums inc = ps_warp_scan(mine, lane);
+        PosSums ex = ps_shfl_up(inc, 1);
         if (lane == 0) possums_zero(ex);
         if (lane == 31) s_w[warp] = inc;
         __syncthreads();
         if (warp == 0) {
             PosSums w;
             if (lane < PP_THREADS / 32) w = s_w[lane]; else possums_zero(w);
-            const PosSums wi = ONE ? ps_warp_scan_one(w, lane) : ps_warp_scan(w, lane);
-            PosSums we = ONE ? ps_shfl_up_one(wi, 1) : ps_shfl_up(wi, 1);
+            const PosSums wi = ps_warp_scan(w, lane);
+            PosSums we = ps_shfl_up(wi, 1);
             if (lane == 0) possums_zero(we);
             if (lane < PP_THREADS / 32) s_w[lane] = we;
             if (lane == PP_THREADS / 32 - 1) {
@@ -1051,10 +1006,9 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a
                 if (!FUSED) {
                     // the tile's terminal nodes take the spans of positions [s_slo, s_shi): the
                     // first terminal index after the last head before the tile, and after the tile
-                    const PosSums tot = ps_join<ONE>(tp, wi);
-                    // (one document: the last ⊢ is position 0)
-                    s_slo = (ONE ? 0u : (uint32_t)tp.hpos) + 1u + tp.terms;
-                    s_shi = (ONE ? 0u : (uint32_t)tot.hpos) + 1u + tot.terms;
+                    const PosSums tot = ps_combine(tp, wi);
+                    s_slo = (uint32_t)tp.hpos + 1u + tp.terms;
+                    s_shi = (uint32_t)tot.hpos + 1u + tot.terms;
                 }
             }
             if (FUSED) {
@@ -1069,6 +1023,7 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a
                 agg.heads = __shfl_sync(ALP_FULL_MASK, wi.heads, LW);
                 agg.hpos = __shfl_sync(ALP_FULL_MASK, wi.hpos, LW);
                 agg.cls = __shfl_sync(ALP_FULL_MASK, wi.cls, LW);
+                agg.dnodes = __shfl_sync(ALP_FULL_MASK, wi.dnodes, LW);
                 const PosSums pre = ps_lookback(a, tile, agg);
                 if (lane == 0) {
                     s_tp = pre;
@@ -1119,7 +1074,7 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a
         uint32_t kof[PP_ITEMS];
         int32_t depj[PP_ITEMS];
         {
-            PosSums run = ps_join<ONE>(ps_join<ONE>(tp, s_w[warp]), ex);  // before this thread's first position
+            PosSums run = ps_combine(ps_combine(tp, s_w[warp]), ex);  // before this thread's first position
 #pragma unroll
             for (int j = 0; j < PP_ITEMS; ++j) {
                 const long long i = i0 + j;
@@ -1130,10 +1085,9 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a
                 depj[j] = 0;
                 if (i < a.L) {
                     const bool head = (hm >> j) & 1u;
-                    // (one document: every sum before position 0 is zero, the last ⊢ is position 0)
-                    const int32_t dep = (head && !ONE) ? 0 : run.depth;
-                    const long long doc = ONE ? 0 : (long long)run.heads + (head ? 1 : 0) - 1;
-                    const bool dok = ONE || (doc >= 0 && doc < a.n_docs);
+                    const int32_t dep = head ? 0 : run.depth;
+                    const long long doc = (long long)run.heads + (head ? 1 : 0) - 1;
+                    const bool dok = doc >= 0 && doc < a.n_docs;
                     depj[j] = dep;
                     // the previous position's top lefts against this position's first rights
                     const uint32_t pid_prev = j == 0 ? prev_id : (uint32_t)ids[j - 1];
@@ -1160,18 +1114,16 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a
                     } else {
                         const PairInfo pi = s_pi[ids[j]];
                         s_pos[ex_slot(pl)] =
-                            ONE ? make_int4((int32_t)pi.prod_begin - (int32_t)nof[j], run.v, (int32_t)(1u + run.terms), dep)
-                                : make_int4((int32_t)pi.prod_begin - (int32_t)nof[j], head ? 0 : run.v,
-                                            (int32_t)((uint32_t)(head ? i : run.hpos) + 1u + (head ? 0u : run.terms)),
-                                            dep);
+                            make_int4((int32_t)pi.prod_begin - (int32_t)nof[j], head ? 0 : run.v,
+                                      (int32_t)((uint32_t)(head ? i : run.hpos) + 1u + (head ? 0u : run.terms)), dep);
                         if (dep + (int32_t)pi.min_ds < 0 && dok) a.doc_valid[doc] = 0;  // depth below zero
-                        e.nodes = pi.n_prod; e.brs = pi.n_br; e.depth = pi.d_depth; e.v = pi.d_v; e.terms = pi.n_term;
+                        e.nodes = pi.n_prod; e.dnodes = pi.n_prod; e.brs = pi.n_br; e.depth = pi.d_depth; e.v = pi.d_v; e.terms = pi.n_term;
                         cnt[j] = (uint32_t)pi.n_prod | ((uint32_t)pi.n_br << 16);
                     }
                     if (((em >> j) & 1u) && (dep + e.depth != 0) && dok) a.doc_valid[doc] = 0;  // unbalanced at the end
-                    if (head && !ONE) { e.heads = 1; e.hpos = (int32_t)i; }
+                    if (head) { e.heads = 1; e.hpos = (int32_t)i; }
                     e.cls = m;
-                    run = ps_join<ONE>(run, e);
+                    run = ps_combine(run, e);
                 }
             }
         }

@@ -338,6 +338,7 @@ def _kernel_alg_bytes(name, units, parse_layout=True):
     # one document: the expansion takes its ⊢ / ⊣ from the position, so it reads no terminal ids
     ids_in = 2 * L if units.get("one_doc") else 4 * L
     table = {
+        "parse_tree_kernel": ids_in + 8 * m + 29 * N,          # ids in, spans in, the nodes out
         "parse_expand_kernel": ids_in + 8 * m + 25 * N + 8 * K,  # ids in, spans in, node fields + kept brackets out
         "parse_expand_kernel(fused)": 2 * L + 8 * m + 25 * N + 8 * K,  # terminals in (keys), spans in, same out
         "lex3_tok_kernel": n + c + tok * m,                    # bytes and chunk states in, tokens out
