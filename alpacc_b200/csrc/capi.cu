@@ -20,6 +20,7 @@
 #include "host_pool.h"
 #include "lexer.cuh"
 #include "lex3.cuh"
+#include "lexwalk.cuh"
 #include "parser.cuh"
 #include "tree.cuh"
 #include "mlp.cuh"
@@ -85,7 +86,7 @@ struct alp_ctx {
     size_t lex_smem = 0;
     bool lex3 = false;                    // DFA small enough for the multi-kernel lexer (lex3.cuh)
     Lex3Tables l3{};
-    size_t l3_fold_smem = 0, l3_scan_smem = 0, l3_count_smem = 0, l3_emit_smem = 0;
+    size_t l3_fold_smem = 0, l3_scan_smem = 0, l3_walk_smem = 0, l3_emit_smem = 0;
     // ---- parser tables ----
     bool has_parser = false;
     ParseTables pt{};
@@ -444,6 +445,30 @@ int load_lexer(alp_ctx* ctx, Reader& r) {
                 }
                 ent[(size_t)s * LX_ROW + b] = (uint16_t)v;
             }
+        std::vector<uint8_t> walk(lw_table_bytes(S), 0);
+        for (int s = 0; s < S; ++s)
+            for (int b = 0; b < 256; ++b) {
+                const uint32_t e = ent[(size_t)s * LX_ROW + b];
+                walk[(size_t)s * LW_ROW + b] =
+                    (uint8_t)((e & LX_NEXT) | (e & LX_EMIT ? LW_EMIT : 0) | (e & LX_START ? LW_START : 0));
+            }
+        ctx->l3.slots = LW_SLOTS;
+        for (int b = 0; b < 256; ++b)
+            if (ent[(size_t)1 * LX_ROW + b] & LX_EMIT) ctx->l3.slots = LW_SLOTS_EMPTY;
+        // the fold's steps, with rows for the constant functions; as byte offsets where those fit
+        ctx->l3.fold2 = 2 * ((size_t)E + S) * C1 <= 65536 && C1 <= 128;
+        const uint32_t unit = ctx->l3.fold2 ? 2u * C1 : 1u;
+        std::vector<uint16_t> fstep((((size_t)E + S) * C1 + 7) & ~(size_t)7, 0);
+        for (size_t i = 0; i < (size_t)E * C1; ++i) fstep[i] = (uint16_t)(vstep[i] * unit);
+        for (int s = 0; s < S; ++s)
+            for (int c = 0; c < C1; ++c)
+                fstep[((size_t)E + s) * C1 + c] = (uint16_t)((E + (vcd[(size_t)s * C1 + c] & 0x7fffu)) * unit);
+        std::vector<uint8_t> fcls(256);
+        for (int b = 0; b < 256; ++b) fcls[b] = (uint8_t)(vcls[b] * (ctx->l3.fold2 ? 2 : 1));
+        if ((rc = upload(ctx, walk.data(), walk.size(), &ctx->l3.walk)) ||
+            (rc = upload(ctx, fstep.data(), fstep.size(), &ctx->l3.fstep)) ||
+            (rc = upload(ctx, fcls.data(), fcls.size(), &ctx->l3.fcls)))
+            return rc;
         ctx->l3.cls = ctx->lt.cls;
         ctx->l3.cdelta = ctx->lt.cdelta;
         ctx->l3.step = ctx->lt.step;
@@ -455,7 +480,7 @@ int load_lexer(alp_ctx* ctx, Reader& r) {
         ctx->l3.E = E;
         ctx->l3_fold_smem = lex3_fold_smem(S, C1, E);
         ctx->l3_scan_smem = lex3_scan_smem(S, E);
-        ctx->l3_count_smem = lex3_count_smem(S);
+        ctx->l3_walk_smem = lex3_walk_smem(S, ctx->l3.slots);
         ctx->l3_emit_smem = lex3_emit_smem(S);
         ctx->lex3 = true;
     }
@@ -666,8 +691,9 @@ struct Lex3Run {
     LexSeg sg;
     uint8_t* base;
     size_t o_td, o_ccs;
-    long long tiles, wide, chunks, stiles, nd;
+    long long tiles, wide, chunks, units, stiles, nd;
     int sms;
+    bool walked = false;  // the chunks' masks and rows are there (lex3_walk_kernel)
 };
 
 int scan_g(const alp_ctx* ctx) { return ctx->tune.scan_g ? ctx->tune.scan_g : LS_G; }
@@ -690,18 +716,23 @@ int lex3_grid(alp_ctx* ctx, const Lex3Run& r, const void* k, int threads, size_t
 }
 
 int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long* d_off, long long nd, int sentinels,
-                 void* term, void* start, void* end, long long cap, uint8_t* valid, Lex3Run& r) {
+                 void* term, void* start, void* end, long long cap, uint8_t* valid, Lex3Run& r, bool wide = true) {
     r.tiles = (n + LX_TILE - 1) / LX_TILE;
     r.wide = (n + LX_WIDE - 1) / LX_WIDE;
     r.chunks = (n + LX_CHUNK - 1) / LX_CHUNK;
-    r.stiles = (r.chunks + ls_tile(scan_g(ctx)) - 1) / ls_tile(scan_g(ctx));
+    // units of the state scan: 64 bytes, or single chunks where no walk follows
+    r.units = wide ? (r.chunks + 1) / 2 : r.chunks;
+    r.stiles = (r.units + ls_tile(scan_g(ctx)) - 1) / ls_tile(scan_g(ctx));
     r.nd = nd;
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t o_vec = 256, o_cs = o_vec + al(128 * (size_t)r.stiles), o_f = o_cs + al(8 * (size_t)r.tiles);
     const size_t o_s = o_f + al(2 * (size_t)r.chunks + 64), o_c = o_s + al((size_t)r.chunks + 64);
     r.o_td = o_c + al(2 * (size_t)r.chunks + 64);
     r.o_ccs = r.o_td + al(8 * (size_t)r.tiles);
-    const size_t sbytes = r.o_ccs + al(8 * ((size_t)r.tiles / LT_CHUNK + 2));
+    const size_t o_r = r.o_ccs + al(8 * ((size_t)r.tiles / LT_CHUNK + 2));
+    const size_t o_x = o_r + al(16 * (size_t)r.chunks + 64);
+    const size_t o_us = o_x + al(2 * (size_t)lw_more(ctx->l3.slots) * r.chunks + 64);
+    const size_t sbytes = o_us + al((size_t)r.units + 64);
     int rc;
     if ((rc = grow(ctx, ctx->scratch, sbytes))) return rc;
     uint8_t* base = reinterpret_cast<uint8_t*>(ctx->scratch.p);
@@ -713,9 +744,13 @@ int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long
     a.aligned16 = ((reinterpret_cast<uintptr_t>(d_in) & 15u) == 0) ? 1 : 0;
     a.t = ctx->l3;
     a.n_chunks = r.chunks;
-    a.chunk_f = reinterpret_cast<uint16_t*>(base + o_f);
+    a.n_units = r.units;
+    a.unit_f = reinterpret_cast<uint16_t*>(base + o_f);
     a.chunk_s = base + o_s;
+    a.unit_s = wide ? base + o_us : a.chunk_s;
     a.chunk_c = reinterpret_cast<uint16_t*>(base + o_c);
+    a.chunk_r = base + o_r;
+    a.chunk_x = reinterpret_cast<uint16_t*>(base + o_x);
     a.tile_cs = reinterpret_cast<unsigned long long*>(base + o_cs);
     a.lb_vec = reinterpret_cast<uint32_t*>(base + o_vec);
     a.res = reinterpret_cast<AlpResult*>(base);
@@ -759,28 +794,36 @@ int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long
 int lex3_fold(alp_ctx* ctx, Lex3Run& r) {
     unsigned g1;
     int rc;
-    CK(cudaFuncSetAttribute(lex3_fold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->l3_fold_smem));
-    CK(cudaFuncSetAttribute(lex3_fold_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    if ((rc = lex3_grid(ctx, r, (const void*)lex3_fold_kernel, LX_THREADS, ctx->l3_fold_smem, r.wide, &g1))) return rc;
+    const bool wide = r.units != r.chunks;
+    const void* k = ctx->l3.fold2
+                        ? (wide ? (const void*)lex3_fold_kernel<true, true> : (const void*)lex3_fold_kernel<true, false>)
+                        : (wide ? (const void*)lex3_fold_kernel<false, true> : (const void*)lex3_fold_kernel<false, false>);
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->l3_fold_smem));
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    if ((rc = lex3_grid(ctx, r, k, LX_THREADS, ctx->l3_fold_smem, r.wide, &g1))) return rc;
     mark(ctx, "start");
-    lex3_fold_kernel<<<g1, LX_THREADS, ctx->l3_fold_smem, ctx->stream>>>(r.a, r.sg);
-    CK(cudaGetLastError());
+    {
+        void* args[] = {&r.a, &r.sg};
+        CK(cudaLaunchKernel(k, dim3(g1), dim3(LX_THREADS), args, ctx->l3_fold_smem, ctx->stream));
+    }
     mark(ctx, "lex3_fold_kernel");
     return ALP_OK;
 }
 
-// chunk endomorphisms -> chunk states -> chunk counts and tile counts
+// chunk endomorphisms -> chunk states -> chunk counts, masks and rows, and tile counts
 int lex3_front(alp_ctx* ctx, Lex3Run& r, bool folded = false) {
     unsigned g3;
     int rc;
     if (!folded && (rc = lex3_fold(ctx, r))) return rc;
-    CK(cudaFuncSetAttribute(lex3_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->l3_count_smem));
-    if ((rc = lex3_grid(ctx, r, (const void*)lex3_count_kernel, LX_THREADS, ctx->l3_count_smem, r.wide, &g3)))
+    CK(cudaFuncSetAttribute(lex3_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->l3_walk_smem));
+    CK(cudaFuncSetAttribute(lex3_walk_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    if ((rc = lex3_grid(ctx, r, (const void*)lex3_walk_kernel, LX_THREADS, ctx->l3_walk_smem, r.wide, &g3)))
         return rc;
     if ((rc = lex3_scan(ctx, r))) return rc;
-    lex3_count_kernel<<<g3, LX_THREADS, ctx->l3_count_smem, ctx->stream>>>(r.a, r.sg);
+    lex3_walk_kernel<<<g3, LX_THREADS, ctx->l3_walk_smem, ctx->stream>>>(r.a, r.sg);
     CK(cudaGetLastError());
-    mark(ctx, "lex3_count_kernel");
+    mark(ctx, "lex3_walk_kernel");
+    r.walked = true;
     return ALP_OK;
 }
 
@@ -798,20 +841,23 @@ int lex3_tiles(alp_ctx* ctx, Lex3Run& r) {
 
 template <typename TermT, typename PosT>
 int lex3_emit(alp_ctx* ctx, Lex3Run& r, bool tiles_done = false) {
-    auto k5 = lex3_emit_kernel<TermT, PosT>;
+    const void* k5 = r.walked ? (const void*)lex3_write_kernel<TermT, PosT> : (const void*)lex3_emit_kernel<TermT, PosT>;
+    const size_t sm = r.walked ? lex3_write_smem() : ctx->l3_emit_smem;
     unsigned g5;
     int rc;
-    CK(cudaFuncSetAttribute(k5, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->l3_emit_smem));
+    CK(cudaFuncSetAttribute(k5, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     CK(cudaFuncSetAttribute(k5, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    if ((rc = lex3_grid(ctx, r, (const void*)k5, LX_THREADS, ctx->l3_emit_smem, r.tiles, &g5))) return rc;
+    if ((rc = lex3_grid(ctx, r, k5, LX_THREADS, sm, r.walked ? r.wide : r.tiles, &g5))) return rc;
     mark(ctx, "start");
     if (!tiles_done) {
         if ((rc = lex3_tiles(ctx, r))) return rc;
         mark(ctx, "lex3_tile_reduce+lex3_tile_scan");
     }
-    k5<<<g5, LX_THREADS, ctx->l3_emit_smem, ctx->stream>>>(r.a, r.sg);
-    CK(cudaGetLastError());
-    mark(ctx, "lex3_emit_kernel");
+    {
+        void* args[] = {&r.a, &r.sg};
+        CK(cudaLaunchKernel(k5, dim3(g5), dim3(LX_THREADS), args, sm, ctx->stream));
+    }
+    mark(ctx, r.walked ? "lex3_write_kernel" : "lex3_emit_kernel");
     return ALP_OK;
 }
 
@@ -883,7 +929,8 @@ int lex3_run(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long* d_
              TermT* term, PosT* start, PosT* end, long long cap, uint8_t* valid, long long* total) {
     Lex3Run r;
     int rc;
-    if ((rc = lex3_prepare(ctx, d_in, n, d_off, nd, sentinels, term, start, end, cap, valid, r))) return rc;
+    if ((rc = lex3_prepare(ctx, d_in, n, d_off, nd, sentinels, term, start, end, cap, valid, r, ctx->tune.lex_split != 0)))
+        return rc;
     if (ctx->tune.lex_split) {
         if ((rc = lex3_front(ctx, r))) return rc;
         return lex3_back<TermT, PosT>(ctx, r, total);
@@ -2691,7 +2738,7 @@ int alp_lex_shard_begin(alp_ctx* ctx, const uint8_t* d_in, int64_t n, int64_t po
     const int rows = ctx->E + ctx->S;
     const size_t fsm = (size_t)rows * 32;
     CK(cudaFuncSetAttribute(lex3_fn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm));
-    lex3_fn_kernel<<<blocks, LF_WARPS * 32, fsm, ctx->stream>>>(s->r.a.chunk_f, s->r.chunks, ctx->l3.app8, rows,
+    lex3_fn_kernel<<<blocks, LF_WARPS * 32, fsm, ctx->stream>>>(s->r.a.unit_f, s->r.units, ctx->l3.app8, rows,
                                                                  s->d_fn);
     CK(cudaGetLastError());
     lex3_fn_final_kernel<<<1, 1024, 0, ctx->stream>>>(s->d_fn, blocks, s->d_fn + (size_t)blocks * 32);
@@ -3476,7 +3523,7 @@ static int spec3_lex(alp_ctx* ctx, const uint16_t* wbf, const float* wf32, int n
                 return rc;
         }
         // 2) every block from its predicted state, 3) re-run blocks until every start is exact
-        const size_t smem = ctx->l3_count_smem;
+        const size_t smem = lex3_stage_off(ctx->S);
         CK(cudaFuncSetAttribute(spec3_run_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         CK(cudaFuncSetAttribute(spec3_fixup_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         mark(ctx, "start");
@@ -3943,7 +3990,7 @@ alp_ctx* child_ctx(const alp_ctx* p) {
     c->lex3 = p->lex3;
     c->l3 = p->l3;
     c->l3_fold_smem = p->l3_fold_smem; c->l3_scan_smem = p->l3_scan_smem;
-    c->l3_count_smem = p->l3_count_smem; c->l3_emit_smem = p->l3_emit_smem;
+    c->l3_walk_smem = p->l3_walk_smem; c->l3_emit_smem = p->l3_emit_smem;
     c->has_parser = p->has_parser;
     c->pt = p->pt;
     c->ph = p->ph;

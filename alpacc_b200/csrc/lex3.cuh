@@ -13,19 +13,21 @@
 //                      the chunks of their warp through the apply table in
 //                      shared memory; tiles chain through a decoupled look-back
 //                      on these vectors.  Output: the state entering each chunk.
-//   lex3_count_kernel  the token-end flags and ignore filter (futhark/lexer.fut:
-//                      103-107) as counts: each thread runs the DFA over two
-//                      chunks from their known states with a 256-column table
-//                      whose entries carry the produce/ignore decisions, and
-//                      stores the chunk's token count and last token start.
+//   lex3_walk_kernel   the token-end flags and ignore filter (futhark/lexer.fut:
+//                      103-107): each thread runs the DFA over two chunks from
+//                      their known states with a 256-column table whose entries
+//                      carry the produce/ignore decisions, and stores the chunk's
+//                      token count, last token start and a record per token
+//                      (lexwalk.cuh).
 //   lex3_tile_reduce_kernel, lex3_tile_scan_kernel  exclusive (count, last
 //                      start) over 8 KiB tiles, the
 //                      take_right start scan and the compaction offsets
 //                      (futhark/lexer.fut:83-84,108-120) at tile level.
-//   lex3_emit_kernel   the compaction (futhark/lexer.fut:121-133): places each
-//                      thread from the stored counts, runs the DFA once more,
-//                      stages the tile's tokens in shared memory and writes
-//                      them with coalesced stores.
+//   lex3_write_kernel  the compaction (futhark/lexer.fut:121-133): places each
+//                      thread from the stored counts and writes the tokens
+//                      from the records (lexwalk.cuh).
+//   lex3_emit_kernel   the same by a second DFA walk: for the speculative lexer,
+//                      whose front end stores counts only.
 #pragma once
 #include "common.cuh"
 #include "lexer.cuh"
@@ -35,7 +37,7 @@ namespace alp {
 constexpr int LX_THREADS = 256;
 constexpr int LX_CHUNK = 32;                    // bytes per chunk, the unit of the state scan
 constexpr int LX_TILE = LX_THREADS * LX_CHUNK;  // 8 KiB emit tile: one chunk per thread
-constexpr int LX_WIDE = 2 * LX_TILE;            // 16 KiB fold / count tile: two chunks per thread
+constexpr int LX_WIDE = 2 * LX_TILE;            // 16 KiB fold / walk tile: two chunks per thread
 constexpr int LX_STAGE = 2048;                  // tokens one emit tile stages in shared memory
 constexpr int LS_WARPS = 8;
 constexpr int LS_G = 16;                        // chunks per lane in the state scan (default; 8, 16 or 32)
@@ -58,6 +60,11 @@ struct Lex3Tables {
                               // identity beyond S in rows < E
     const uint16_t* ent;      // [S][LX_ROW] next | LX_START | LX_EMIT | term << LX_TERM_SHIFT (columns 256.. unused)
     const uint32_t* tokinfo;  // [S] terminal | TOK_ACCEPT | TOK_IGNORE
+    const uint8_t* walk;      // [S][LW_ROW] the walk table (lexwalk.cuh)
+    const uint16_t* fstep;    // [E+S][C1] the fold's steps (rows E+s: the constant function s); see fold2
+    const uint8_t* fcls;      // [256] byte -> class as fstep counts it
+    int fold2;                // 1: fstep holds 2 * C1 * next and fcls 2 * class; 0: next and class
+    int slots;                // records a chunk can have (lexwalk.cuh)
     int S, C1, E;
 };
 
@@ -80,9 +87,13 @@ struct Lex3Args {
     int aligned16;
     Lex3Tables t;
     long long n_chunks;            // ceil(n / 32)
-    uint16_t* chunk_f;             // [n_chunks] endomorphism of each chunk (E + s: constant s)
-    uint8_t* chunk_s;              // [n_chunks] state entering each chunk
+    long long n_units;             // units of the state scan: chunks, or pairs of chunks (64 bytes)
+    uint16_t* unit_f;              // [n_units] endomorphism of each unit (E + s: constant s)
+    uint8_t* unit_s;               // [n_units] state entering each unit
+    uint8_t* chunk_s;              // [n_chunks] state entering each chunk (unit_s where units are chunks)
     uint16_t* chunk_c;             // [n_chunks] tokens ending in the chunk | last start offset << 8
+    uint8_t* chunk_r;              // [n_chunks][16] records of its first eight tokens (lexwalk.cuh)
+    uint16_t* chunk_x;             // [n_chunks][lw_more(t.slots)] and of the others
     unsigned long long* tile_cs;   // [tiles] count << 32 | last start; inclusive per tile, then exclusive
     uint32_t* lb_vec;              // [scan tiles][32] state-scan look-back words
     unsigned int* tickets;         // [0] state scan
@@ -102,17 +113,13 @@ struct Lex3Args {
 };
 
 __host__ __device__ inline size_t lex3_fold_smem(int S, int C1, int E) {
-    size_t b = 256 + 2 * (size_t)S * C1;
-    b = (b + 15) & ~(size_t)15;
-    b += 2 * (size_t)E * C1;
-    return (b + 15) & ~(size_t)15;
+    return (256 + 2 * ((size_t)E + S) * C1 + 15) & ~(size_t)15;
 }
 __host__ __device__ inline size_t lex3_scan_smem(int S, int E) {
     return (32 * ((size_t)E + S) + 15) & ~(size_t)15;
 }
 __host__ __device__ inline size_t lex3_tok_off(int S) { return (2 * (size_t)S * LX_ROW + 15) & ~(size_t)15; }
 __host__ __device__ inline size_t lex3_stage_off(int S) { return (lex3_tok_off(S) + 4 * (size_t)S + 15) & ~(size_t)15; }
-__host__ __device__ inline size_t lex3_count_smem(int S) { return lex3_stage_off(S); }
 __host__ __device__ inline size_t lex3_emit_smem(int S) { return lex3_stage_off(S) + (size_t)LX_STAGE * 8; }
 
 template <int NV>
@@ -158,12 +165,42 @@ __device__ __forceinline__ void lx_mark_docs(const LexSeg& sg, long long n, long
     }
 }
 
+// 16*NV bytes from NV + 1 aligned words of 16, W words and `bits` bits into the first.
+template <int NV, int W>
+__device__ __forceinline__ void lx_shift(const uint32_t (&x)[4 * NV + 4], uint32_t bits, uint4 (&w)[NV]) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        uint32_t y[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) y[q] = __funnelshift_r(x[4 * v + q + W], 4 * v + q + W + 1 < 4 * NV + 4 ? x[4 * v + q + W + 1] : 0u, bits);
+        w[v] = make_uint4(y[0], y[1], y[2], y[3]);
+    }
+}
+
 // The (up to) 16*NV bytes starting at `my`.
 template <int NV>
 __device__ __forceinline__ void lx_load(const Lex3Args& a, long long my, int lim, uint4 (&w)[NV]) {
     if (a.aligned16 && lim == 16 * NV) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) w[v] = __ldg(reinterpret_cast<const uint4*>(a.in + my) + v);
+    } else if (my >= 16 && my + 16 * NV + 16 <= a.n) {
+        // an input off a 16-byte boundary: the aligned words around the bytes (all inside
+        // the input), shifted into place
+        const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(a.in) & 15u);
+        const uint4* p = reinterpret_cast<const uint4*>(a.in + my - sh);
+        uint32_t x[4 * NV + 4];
+#pragma unroll
+        for (int v = 0; v <= NV; ++v) {
+            const uint4 y = __ldg(p + v);
+            x[4 * v] = y.x; x[4 * v + 1] = y.y; x[4 * v + 2] = y.z; x[4 * v + 3] = y.w;
+        }
+        const uint32_t bits = 8u * (sh & 3u);
+        switch (sh >> 2) {
+            case 0: lx_shift<NV, 0>(x, bits, w); break;
+            case 1: lx_shift<NV, 1>(x, bits, w); break;
+            case 2: lx_shift<NV, 2>(x, bits, w); break;
+            default: lx_shift<NV, 3>(x, bits, w); break;
+        }
     } else {
         uint32_t x[4 * NV];
 #pragma unroll
@@ -181,38 +218,66 @@ __device__ __forceinline__ void lx_load(const Lex3Args& a, long long my, int lim
 
 // ---- kernel 1: chunk endomorphisms ------------------------------------------
 
-// One chunk's endomorphism from bytes in[0, lim), with document heads (a
-// compact loop: only chunks at document heads or the input's end).
-__device__ __forceinline__ uint32_t lx_fold_slow(const uint8_t* in, int lim, uint32_t head,
-                                                 const uint8_t* s_cls, const uint16_t* s_cd, const uint16_t* s_step,
-                                                 int C1, uint32_t E) {
-    uint32_t f = 0;
+// Up to eight bytes at p (lim of them), all loads in flight at once.
+__device__ __forceinline__ unsigned long long lx_bytes8(const uint8_t* p, int lim) {
+    uint32_t x[8];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) x[b] = b < lim ? (uint32_t)__ldg(p + b) : 0u;
+    const uint32_t lo = x[0] | (x[1] << 8) | (x[2] << 16) | (x[3] << 24);
+    const uint32_t hi = x[4] | (x[5] << 8) | (x[6] << 16) | (x[7] << 24);
+    return ((unsigned long long)hi << 32) | lo;
+}
+
+// One step of the fold: f stands for an endomorphism as fstep holds it.  With F2 both
+// table values are byte offsets already: a step is one addition beside its two lookups.
+template <bool F2>
+__device__ __forceinline__ uint32_t lx_step(const uint8_t* s_step, const uint8_t* s_cls, uint32_t f, uint32_t b, int C1) {
+    const uint32_t at = F2 ? f + s_cls[b] : 2u * (f * (uint32_t)C1 + s_cls[b]);
+    return *reinterpret_cast<const uint16_t*>(s_step + at);
+}
+
+// The endomorphism f and then bytes in[0, lim), with document heads: only threads at
+// document heads or the input's end.  `init`: the constant function of the initial state.
+template <bool F2>
+__device__ __forceinline__ uint32_t lx_fold_slow(const uint8_t* in, int lim, unsigned long long head, uint32_t f,
+                                                 const uint8_t* s_cls, const uint8_t* s_step, int C1, uint32_t init) {
 #pragma unroll 1
-    for (int j = 0; j < lim; ++j) {
-        {
-            const uint32_t c = s_cls[__ldg(in + j)];
-            if ((head >> j) & 1u) f = E + (s_cd[1 * C1 + c] & 0x7fffu);
-            else if (f >= E) f = E + (s_cd[(f - E) * C1 + c] & 0x7fffu);
-            else f = s_step[f * C1 + c];
+    for (int j0 = 0; j0 < lim; j0 += 8) {
+        const unsigned long long w = lx_bytes8(in + j0, lim - j0);
+        const int e8 = min(8, lim - j0);
+#pragma unroll 1
+        for (int i = 0; i < e8; ++i) {
+            if ((head >> (j0 + i)) & 1ull) f = init;
+            f = lx_step<F2>(s_step, s_cls, f, (uint32_t)(w >> (8 * i)) & 0xffu, C1);
         }
     }
     return f;
 }
 
+// WIDE: a unit is a thread's 64 bytes, folded as one chain; else its two chunks, side by side.
+template <bool F2, bool WIDE>
 __global__ void __launch_bounds__(LX_THREADS, 4) lex3_fold_kernel(Lex3Args a, LexSeg sg) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int S = a.t.S, C1 = a.t.C1;
     const uint32_t E = (uint32_t)a.t.E;
     uint8_t* s_cls = smem;
-    uint16_t* s_cd = reinterpret_cast<uint16_t*>(smem + 256);
-    const size_t off_step = (256 + 2 * (size_t)S * C1 + 15) & ~(size_t)15;
-    uint16_t* s_step = reinterpret_cast<uint16_t*>(smem + off_step);
+    uint8_t* s_step = smem + 256;
     __shared__ uint32_t s_head[LX_WIDE / LX_CHUNK];
 
     const int tid = threadIdx.x;
-    for (int i = tid; i < 256; i += LX_THREADS) s_cls[i] = a.t.cls[i];
-    for (int i = tid; i < S * C1; i += LX_THREADS) s_cd[i] = a.t.cdelta[i];
-    for (int i = tid; i < (int)E * C1; i += LX_THREADS) s_step[i] = a.t.step[i];
+    {
+        // (the uploaded tables are padded to whole 16-byte words)
+        const uint4* src = reinterpret_cast<const uint4*>(a.t.fcls);
+        for (int i = tid; i < 16; i += LX_THREADS) reinterpret_cast<uint4*>(s_cls)[i] = __ldg(src + i);
+        src = reinterpret_cast<const uint4*>(a.t.fstep);
+        const int words = (int)((2 * (size_t)(E + S) * C1 + 15) / 16);
+        for (int i = tid; i < words; i += LX_THREADS) reinterpret_cast<uint4*>(s_step)[i] = __ldg(src + i);
+    }
+    const uint32_t unit = F2 ? 2u * (uint32_t)C1 : 1u;
+    const uint32_t init = (E + 1u) * unit;
+    // endomorphism number of a fold value: exact for values below 2^16 (umulhi by ceil(2^32 / unit))
+    const uint32_t inv = F2 ? (uint32_t)((0x100000000ull + unit - 1) / unit) : 0u;
+    auto number = [&](uint32_t f) -> uint32_t { return F2 ? __umulhi(f, inv) : f; };
     const long long n = a.n;
     // this thread's 64 bytes of a tile, one tile ahead (in flight while the block folds
     // the tile before)
@@ -220,7 +285,7 @@ __global__ void __launch_bounds__(LX_THREADS, 4) lex3_fold_kernel(Lex3Args a, Le
     auto tile_bytes = [&](unsigned ft, uint4 (&w)[4]) {
         const long long my = (long long)ft * LX_WIDE + (long long)tid * (2 * LX_CHUNK);
         const int lim = (int)max(0ll, min((long long)(2 * LX_CHUNK), n - my));
-        if (lim > 0) lx_load<4>(a, my, lim, w);
+        if (lim == 2 * LX_CHUNK) lx_load<4>(a, my, lim, w);
     };
     if (blockIdx.x < a.num_wide) tile_bytes(blockIdx.x, nw);
     for (unsigned ft = blockIdx.x; ft < a.num_wide; ft += gridDim.x) {
@@ -238,19 +303,28 @@ __global__ void __launch_bounds__(LX_THREADS, 4) lex3_fold_kernel(Lex3Args a, Le
         if (lim > 0) {
             const uint32_t ha = s_head[2 * tid], hb = s_head[2 * tid + 1];
             const long long c = my / LX_CHUNK;
-            if (lim == 2 * LX_CHUNK && (ha | hb) == 0) {
+            if (WIDE) {
+                uint32_t f = 0;
+                if (lim == 2 * LX_CHUNK && (ha | hb) == 0) {
+#pragma unroll
+                    for (int j = 0; j < 2 * LX_CHUNK; ++j) f = lx_step<F2>(s_step, s_cls, f, byte_of(w, j), C1);
+                } else {
+                    f = lx_fold_slow<F2>(a.in + my, lim, ha | ((unsigned long long)hb << 32), 0, s_cls, s_step, C1, init);
+                }
+                a.unit_f[my / (2 * LX_CHUNK)] = (uint16_t)number(f);
+            } else if (lim == 2 * LX_CHUNK && (ha | hb) == 0) {
                 uint32_t fa = 0, fb = 0;
 #pragma unroll
                 for (int j = 0; j < LX_CHUNK; ++j) {
-                    fa = s_step[fa * C1 + s_cls[byte_of(w, j)]];
-                    fb = s_step[fb * C1 + s_cls[byte_of(w, LX_CHUNK + j)]];
+                    fa = lx_step<F2>(s_step, s_cls, fa, byte_of(w, j), C1);
+                    fb = lx_step<F2>(s_step, s_cls, fb, byte_of(w, LX_CHUNK + j), C1);
                 }
-                *reinterpret_cast<uint32_t*>(a.chunk_f + c) = fa | (fb << 16);
+                *reinterpret_cast<uint32_t*>(a.unit_f + c) = number(fa) | (number(fb) << 16);
             } else {
-                a.chunk_f[c] = (uint16_t)lx_fold_slow(a.in + my, min(lim, LX_CHUNK), ha, s_cls, s_cd, s_step, C1, E);
+                a.unit_f[c] = (uint16_t)number(lx_fold_slow<F2>(a.in + my, min(lim, LX_CHUNK), ha, 0, s_cls, s_step, C1, init));
                 if (lim > LX_CHUNK)
-                    a.chunk_f[c + 1] =
-                        (uint16_t)lx_fold_slow(a.in + my + LX_CHUNK, lim - LX_CHUNK, hb, s_cls, s_cd, s_step, C1, E);
+                    a.unit_f[c + 1] = (uint16_t)number(
+                        lx_fold_slow<F2>(a.in + my + LX_CHUNK, lim - LX_CHUNK, hb, 0, s_cls, s_step, C1, init));
             }
         }
         __syncthreads();
@@ -277,7 +351,7 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
         for (uint32_t i = tid; i < rows * 2; i += LS_WARPS * 32) dst[i] = src[i];
     }
     const uint32_t INIT = 1u;
-    const long long M = a.n_chunks;
+    const long long M = a.n_units;
     for (;;) {
         if (tid == 0) s_tile = atomicAdd(&a.tickets[0], 1u);
         __syncthreads();
@@ -288,7 +362,7 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
         // this lane's G chunk endomorphisms, two per word
         uint32_t fr[G / 2];
         if (base + G <= M) {
-            const uint4* p = reinterpret_cast<const uint4*>(a.chunk_f + base);
+            const uint4* p = reinterpret_cast<const uint4*>(a.unit_f + base);
 #pragma unroll
             for (int v = 0; v < G / 8; ++v) {
                 const uint4 x = p[v];
@@ -297,8 +371,8 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
         } else {
 #pragma unroll
             for (int q = 0; q < G / 2; ++q) {
-                const uint32_t lo = base + 2 * q < M ? a.chunk_f[base + 2 * q] : 0u;
-                const uint32_t hi = base + 2 * q + 1 < M ? a.chunk_f[base + 2 * q + 1] : 0u;
+                const uint32_t lo = base + 2 * q < M ? a.unit_f[base + 2 * q] : 0u;
+                const uint32_t hi = base + 2 * q + 1 < M ? a.unit_f[base + 2 * q + 1] : 0u;
                 fr[q] = lo | (hi << 16);
             }
         }
@@ -376,17 +450,17 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
         }
         if (base + G <= M) {
             if constexpr (G == 8) {
-                *reinterpret_cast<uint2*>(a.chunk_s + base) = make_uint2(ob[0], ob[1]);
+                *reinterpret_cast<uint2*>(a.unit_s + base) = make_uint2(ob[0], ob[1]);
             } else {
 #pragma unroll
                 for (int v = 0; v < G / 16; ++v)
-                    reinterpret_cast<uint4*>(a.chunk_s + base)[v] =
+                    reinterpret_cast<uint4*>(a.unit_s + base)[v] =
                         make_uint4(ob[4 * v], ob[4 * v + 1], ob[4 * v + 2], ob[4 * v + 3]);
             }
         } else {
 #pragma unroll
             for (int g = 0; g < G; ++g)
-                if (base + g < M) a.chunk_s[base + g] = (uint8_t)(ob[g >> 2] >> (8 * (g & 3)));
+                if (base + g < M) a.unit_s[base + g] = (uint8_t)(ob[g >> 2] >> (8 * (g & 3)));
         }
         __syncthreads();
     }
@@ -400,14 +474,18 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
 // without one).  A compact loop: only chunks at document boundaries or the
 // input's end.
 __device__ __forceinline__ uint32_t lx_count_slow(const uint8_t* in, int lim, uint32_t st, uint32_t head,
-                                                  uint32_t last, const uint16_t* s_ent, const uint32_t* s_tok,
+                                                  uint32_t last, const uint16_t* ent, const uint32_t* s_tok,
                                                   uint32_t* lastoff, uint32_t* endinfo) {
     uint32_t cnt = 0, lo = LX_NOOFF;
 #pragma unroll 1
-    for (int j = 0; j < lim; ++j) {
-        {
+    for (int j0 = 0; j0 < lim; j0 += 8) {
+        const unsigned long long w = lx_bytes8(in + j0, lim - j0);
+        const int e8 = min(8, lim - j0);
+#pragma unroll 1
+        for (int i = 0; i < e8; ++i) {
+            const int j = j0 + i;
             if ((head >> j) & 1u) { st = 1u; lo = (uint32_t)j; }
-            const uint32_t e = s_ent[st * LX_ROW + __ldg(in + j)];
+            const uint32_t e = ent[st * LX_ROW + ((uint32_t)(w >> (8 * i)) & 0xffu)];
             cnt += (e >> 6) & 1u;
             if (e & LX_START) lo = (uint32_t)j;
             st = e & LX_NEXT;
@@ -430,93 +508,6 @@ __device__ __forceinline__ void cs_reduce_warp(uint32_t& c, uint32_t& p) {
         const uint32_t op = __shfl_down_sync(ALP_FULL_MASK, p, d);
         c += oc;
         if (op != ALP_NONE32) p = op;
-    }
-}
-
-__global__ void __launch_bounds__(LX_THREADS, 6) lex3_count_kernel(Lex3Args a, LexSeg sg) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    const int S = a.t.S;
-    uint16_t* s_ent = reinterpret_cast<uint16_t*>(smem);
-    uint32_t* s_tok = reinterpret_cast<uint32_t*>(smem + lex3_tok_off(S));
-    __shared__ uint32_t s_head[LX_WIDE / LX_CHUNK], s_last[LX_WIDE / LX_CHUNK];
-    __shared__ uint32_t s_wc[LX_THREADS / 32], s_wp[LX_THREADS / 32];
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    {
-        const uint4* src = reinterpret_cast<const uint4*>(a.t.ent);
-        uint4* dst = reinterpret_cast<uint4*>(s_ent);
-        for (int i = tid; i < (S * LX_ROW * 2 + 15) / 16; i += LX_THREADS) dst[i] = src[i];
-    }
-    for (int i = tid; i < S; i += LX_THREADS) s_tok[i] = a.t.tokinfo[i];
-    const long long n = a.n;
-    for (unsigned ft = blockIdx.x; ft < a.num_wide; ft += gridDim.x) {
-        const long long t0 = (long long)ft * LX_WIDE;
-        const long long t1 = min(t0 + LX_WIDE, n) - 1;
-        s_head[tid] = 0;
-        s_head[tid + LX_THREADS] = 0;
-        s_last[tid] = 0;
-        s_last[tid + LX_THREADS] = 0;
-        __syncthreads();
-        lx_mark_docs(sg, n, sg.n_docs > 1 ? a.tile_doc[2 * (size_t)ft] : 0, t0, t1, s_head, s_last, nullptr);
-        __syncthreads();
-        const long long my = t0 + (long long)tid * (2 * LX_CHUNK);
-        const int lim = (int)max(0ll, min((long long)(2 * LX_CHUNK), n - my));
-        uint32_t cnt = 0, lastp = ALP_NONE32;
-        if (lim > 0) {
-            uint4 w[4];
-            lx_load<4>(a, my, lim, w);
-            const long long c = my / LX_CHUNK;
-            const uint32_t ha = s_head[2 * tid], hb = s_head[2 * tid + 1];
-            const uint32_t la = s_last[2 * tid], lb = s_last[2 * tid + 1];
-            uint32_t ca, cb = 0, oa, ob = LX_NOOFF;
-            if (lim == 2 * LX_CHUNK && (ha | hb | la | lb) == 0) {
-                const uint32_t sab = *reinterpret_cast<const uint16_t*>(a.chunk_s + c);
-                uint32_t sa = sab & 0xffu, sb = sab >> 8;
-                ca = 0;
-                oa = LX_NOOFF;
-#pragma unroll
-                for (int j = 0; j < LX_CHUNK; ++j) {
-                    const uint32_t ea = s_ent[sa * LX_ROW + byte_of(w, j)];
-                    const uint32_t eb = s_ent[sb * LX_ROW + byte_of(w, LX_CHUNK + j)];
-                    ca += (ea >> 6) & 1u;
-                    cb += (eb >> 6) & 1u;
-                    if (ea & LX_START) oa = (uint32_t)j;
-                    if (eb & LX_START) ob = (uint32_t)j;
-                    sa = ea & LX_NEXT;
-                    sb = eb & LX_NEXT;
-                }
-                *reinterpret_cast<uint32_t*>(a.chunk_c + c) = (ca | (oa << 8)) | ((cb | (ob << 8)) << 16);
-            } else {
-                uint32_t ei = 0;
-                ca = lx_count_slow(a.in + my, min(lim, LX_CHUNK), a.chunk_s[c], ha, la, s_ent, s_tok, &oa, &ei);
-                a.chunk_c[c] = (uint16_t)(ca | (oa << 8));
-                if (lim > LX_CHUNK) {
-                    cb = lx_count_slow(a.in + my + LX_CHUNK, lim - LX_CHUNK, a.chunk_s[c + 1], hb, lb, s_ent, s_tok,
-                                       &ob, &ei);
-                    a.chunk_c[c + 1] = (uint16_t)(cb | (ob << 8));
-                }
-                // one document: accepted or not, known before its tokens are written
-                if (sg.n_docs == 1 && (la | lb)) a.res->aux[7] = (ei & TOK_ACCEPT) ? 1 : 0;
-            }
-            cnt = ca + cb;
-            lastp = ob != LX_NOOFF ? (uint32_t)(my + LX_CHUNK + ob)
-                                   : (oa != LX_NOOFF ? (uint32_t)(my + oa) : ALP_NONE32);
-        }
-        // per 8 KiB tile (threads 0..127 and 128..255): count and last start
-        cs_reduce_warp(cnt, lastp);
-        if (lane == 0) { s_wc[warp] = cnt; s_wp[warp] = lastp; }
-        __syncthreads();
-        if (tid == 0 || tid == LX_THREADS / 2) {
-            const int w0 = tid / 32;
-            uint32_t c = 0, p = ALP_NONE32;
-            for (int w2 = w0; w2 < w0 + LX_THREADS / 64; ++w2) {
-                c += s_wc[w2];
-                if (s_wp[w2] != ALP_NONE32) p = s_wp[w2];
-            }
-            const size_t t8 = 2 * (size_t)ft + (tid ? 1 : 0);
-            if (t8 < a.num_tiles) a.tile_cs[t8] = ((unsigned long long)c << 32) | p;
-        }
-        __syncthreads();
     }
 }
 
@@ -832,8 +823,8 @@ __global__ void __launch_bounds__(LX_THREADS, 6) lex3_emit_kernel(Lex3Args a, Le
 }
 
 // ---- kernel 3+4+5 fused: counts, look-back over tiles, tokens ---------------
-// One pass over the input for what lex3_count_kernel, the tile scan and
-// lex3_emit_kernel do in three: each thread runs the DFA over its chunk once
+// One pass over the input for what lex3_walk_kernel, the tile scan and
+// lex3_write_kernel do in three: each thread runs the DFA over its chunk once
 // from its known state, counting the tokens that end in it and keeping each
 // token's place and terminal as a record in shared memory; a block scan places
 // the threads in the tile; the tile publishes its (count, last start) and
@@ -1247,7 +1238,7 @@ __global__ void lex3_stream_end_kernel(LexCarry* c, const uint32_t* tokinfo, lon
 // warp per sub-run, then the warps in order); lex3_fn_final_kernel composes
 // the blocks in order.
 constexpr int LF_WARPS = 8;
-__global__ void __launch_bounds__(LF_WARPS * 32) lex3_fn_kernel(const uint16_t* chunk_f, long long C,
+__global__ void __launch_bounds__(LF_WARPS * 32) lex3_fn_kernel(const uint16_t* unit_f, long long C,
                                                                 const uint8_t* app8, int rows, uint8_t* fn) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint8_t s_w[LF_WARPS][32];
@@ -1263,7 +1254,7 @@ __global__ void __launch_bounds__(LF_WARPS * 32) lex3_fn_kernel(const uint16_t* 
     const long long per_warp = (b1 - b0 + LF_WARPS - 1) / LF_WARPS;
     const long long w0 = b0 + (long long)warp * per_warp, w1 = min(b1, w0 + per_warp);
     uint32_t cur = (uint32_t)lane;
-    for (long long c = w0; c < w1; ++c) cur = smem[(uint32_t)chunk_f[c] * 32 + cur];
+    for (long long c = w0; c < w1; ++c) cur = smem[(uint32_t)unit_f[c] * 32 + cur];
     s_w[warp][lane] = (uint8_t)cur;
     __syncthreads();
     if (warp == 0) {

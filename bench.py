@@ -345,8 +345,9 @@ def _kernel_alg_bytes(name, units, parse_layout=True):
         "ple_tile_kernel(nodes)": 12 * N,                      # values in, parents out
         "ple_tile_kernel(brackets)": 8 * K,                    # kept brackets' depth values and symbols in
         "lex3_emit_kernel": n + 3 * c + tok * m,               # bytes, chunk states and counts in, tokens out
-        "lex3_fold_kernel": n + 2 * c,                         # bytes in, chunk endomorphisms out
-        "lex3_count_kernel": n + 3 * c,                        # bytes, chunk states in, counts out
+        "lex3_write_kernel": 2 * c + 2 * m + tok * m,          # chunk counts and token records in, tokens out
+        "lex3_fold_kernel": n + c,                             # bytes in, an endomorphism per 64 bytes out
+        "lex3_walk_kernel": n + c // 2 + 3 * c + 2 * m,        # bytes, states in, chunk states, counts and records out
         "parse_pairs_kernel": 4 * L,                           # terminal ids in, pair ids out
     }
     return table.get(name)
