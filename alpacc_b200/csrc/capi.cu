@@ -157,6 +157,20 @@ struct alp_ctx {
     DevBuf carry;
     LexCarry* h_carry = nullptr;          // pinned, [2]
     Tuning tune;
+    // CTAs per SM of each kernel at a dynamic shared size, and the kernels whose attributes are set
+    struct Fit {
+        const void* fn;
+        size_t smem;
+        int threads, per_sm;
+    };
+    std::vector<Fit> fits;
+    struct SpanFit {  // expand / tree launches: token spans that fit, and the shared memory with them
+        const void* fn;
+        size_t base, sm;
+        int ctas, span_cap;
+    };
+    std::vector<SpanFit> span_fits;
+    int sms = 0, sm_smem = 0, sm_reserved = 0, sm_optin = 0;
 };
 
 struct alp_lex_stream {
@@ -292,6 +306,36 @@ int send_to_host(alp_ctx* ctx, cudaStream_t s) {
     const cudaError_t e = cudaStreamSynchronize(s);
     if (!rc && e != cudaSuccess) rc = fail(ctx, ALP_ERR_CUDA, "copy to the host: %s", cudaGetErrorString(e));
     return rc;
+}
+
+int device_limits(alp_ctx* ctx) {
+    if (ctx->sms) return ALP_OK;
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&ctx->sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device));
+    CK(cudaDeviceGetAttribute(&ctx->sm_reserved, cudaDevAttrReservedSharedMemoryPerBlock, ctx->device));
+    CK(cudaDeviceGetAttribute(&ctx->sm_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    ctx->sms = sms;
+    return ALP_OK;
+}
+
+// CTAs per SM of a kernel, asked once per context.  The kernel's dynamic shared limit goes to
+// the device's (the same value from every context: it belongs to the kernel, not the call).
+int fit_blocks(alp_ctx* ctx, const void* fn, int threads, size_t smem, bool carveout, int* per_sm) {
+    for (const alp_ctx::Fit& f : ctx->fits)
+        if (f.fn == fn && f.smem == smem && f.threads == threads) {
+            *per_sm = f.per_sm;
+            return ALP_OK;
+        }
+    int rc;
+    if ((rc = device_limits(ctx))) return rc;
+    cudaFuncAttributes fa;
+    CK(cudaFuncGetAttributes(&fa, fn));
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->sm_optin - (int)fa.sharedSizeBytes));
+    if (carveout) CK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, threads, smem));
+    ctx->fits.push_back({fn, smem, threads, *per_sm});
+    return ALP_OK;
 }
 
 int grow(alp_ctx* ctx, DevBuf& b, size_t bytes) {
@@ -682,6 +726,13 @@ int run_ple(alp_ctx* ctx, const int32_t* val, long long n, const uint32_t* sym, 
     return ALP_OK;
 }
 
+// The head of ctx->scratch, cleared before the kernels of a call: the lexer's result at 0,
+// tickets, the parser's result, one document's validity, then the flags of the two tile
+// scans.  One copy of SC_COPY bytes brings the results and the validity to the host.
+constexpr size_t SC_TICKETS = 128, SC_PARSE = 160, SC_VALID = 240, SC_COPY = 256;
+static_assert(sizeof(AlpResult) <= SC_TICKETS && SC_PARSE + sizeof(AlpResult) <= SC_VALID, "scratch head");
+enum { TK_STATES = 0, TK_TOKENS, TK_LEX_TILES, TK_POS_TILES };
+
 // Multi-kernel lexer (DFAs of at most 32 states): chunk endomorphisms, the
 // state scan over them, token counts, the tile scan of the counts, and the
 // token pass.  Same contract as lex_seg.  Split in stages so that the
@@ -693,7 +744,8 @@ struct Lex3Run {
     size_t o_td, o_ccs;
     long long tiles, wide, chunks, units, stiles, nd;
     int sms;
-    bool walked = false;  // the chunks' masks and rows are there (lex3_walk_kernel)
+    bool walked = false;  // the chunks' token records are there (lex3_walk_kernel)
+    ScanSync lex_sync, pos_sync;  // of the scans over lexer tiles and position tiles
 };
 
 int scan_g(const alp_ctx* ctx) { return ctx->tune.scan_g ? ctx->tune.scan_g : LS_G; }
@@ -707,9 +759,10 @@ inline const void* scan_kernel_for(int g) {
 // the state scan over the chunk endomorphisms, chunks per lane as tuned
 int lex3_scan(alp_ctx* ctx, Lex3Run& r);
 
-int lex3_grid(alp_ctx* ctx, const Lex3Run& r, const void* k, int threads, size_t smem, long long work, unsigned* g) {
-    int per_sm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem));
+int lex3_grid(alp_ctx* ctx, const Lex3Run& r, const void* k, int threads, size_t smem, long long work, unsigned* g,
+              bool carveout = true) {
+    int rc, per_sm = 0;
+    if ((rc = fit_blocks(ctx, k, threads, smem, carveout, &per_sm))) return rc;
     long long x = (long long)(per_sm > 0 ? per_sm : 1) * r.sms;
     *g = (unsigned)(x < work ? x : work);
     return ALP_OK;
@@ -725,7 +778,10 @@ int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long
     r.stiles = (r.units + ls_tile(scan_g(ctx)) - 1) / ls_tile(scan_g(ctx));
     r.nd = nd;
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    const size_t o_vec = 256, o_cs = o_vec + al(128 * (size_t)r.stiles), o_f = o_cs + al(8 * (size_t)r.tiles);
+    // flags of the scans over chunks of lexer tiles and of position tiles
+    const size_t o_lf = SC_COPY, o_pf = o_lf + 4 * ((size_t)r.tiles / LT_CHUNK + 2);
+    const size_t pchunks = (size_t)(n + 2 * nd) / ((size_t)PP_TILE * ST_CHUNK) + 2;
+    const size_t o_vec = al(o_pf + 4 * pchunks), o_cs = o_vec + al(128 * (size_t)r.stiles), o_f = o_cs + al(8 * (size_t)r.tiles);
     const size_t o_s = o_f + al(2 * (size_t)r.chunks + 64), o_c = o_s + al((size_t)r.chunks + 64);
     r.o_td = o_c + al(2 * (size_t)r.chunks + 64);
     r.o_ccs = r.o_td + al(8 * (size_t)r.tiles);
@@ -754,7 +810,9 @@ int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long
     a.tile_cs = reinterpret_cast<unsigned long long*>(base + o_cs);
     a.lb_vec = reinterpret_cast<uint32_t*>(base + o_vec);
     a.res = reinterpret_cast<AlpResult*>(base);
-    a.tickets = reinterpret_cast<unsigned int*>(base + 128);
+    a.tickets = reinterpret_cast<unsigned int*>(base + SC_TICKETS);
+    r.lex_sync = ScanSync{a.tickets + TK_LEX_TILES, reinterpret_cast<uint32_t*>(base + o_lf), base + r.o_ccs};
+    r.pos_sync = ScanSync{a.tickets + TK_POS_TILES, reinterpret_cast<uint32_t*>(base + o_pf), nullptr};
     a.tile_doc = reinterpret_cast<const long long*>(base + r.o_td);
     a.out_term = term;
     a.out_start = start;
@@ -769,7 +827,7 @@ int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long
     a.tok_first = 0;
     LexSeg& sg = r.sg;
     sg.cont = 0;
-    sg.end1 = 0;
+    sg.end1 = n;  // one document without an offsets array (d_off null)
     sg.doc_off = d_off;
     sg.n_docs = nd;
     sg.tok_off = (long long*)ctx->tmp[T_TOKOFF].p;
@@ -777,7 +835,8 @@ int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long
     sg.sentinels = sentinels;
     sg.sent_l = ctx->has_parser ? ctx->pt.start : 0;
     sg.sent_r = ctx->has_parser ? ctx->pt.end : 0;
-    CK(cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    if ((rc = device_limits(ctx))) return rc;
+    r.sms = ctx->sms;
     if (nd > 1) {
         const long long gb = (nd + 255) / 256;
         CK(cudaMemsetAsync(base + r.o_td, 0, 8 * (size_t)r.tiles, ctx->stream));
@@ -798,8 +857,6 @@ int lex3_fold(alp_ctx* ctx, Lex3Run& r) {
     const void* k = ctx->l3.fold2
                         ? (wide ? (const void*)lex3_fold_kernel<true, true> : (const void*)lex3_fold_kernel<true, false>)
                         : (wide ? (const void*)lex3_fold_kernel<false, true> : (const void*)lex3_fold_kernel<false, false>);
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->l3_fold_smem));
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     if ((rc = lex3_grid(ctx, r, k, LX_THREADS, ctx->l3_fold_smem, r.wide, &g1))) return rc;
     mark(ctx, "start");
     {
@@ -815,8 +872,6 @@ int lex3_front(alp_ctx* ctx, Lex3Run& r, bool folded = false) {
     unsigned g3;
     int rc;
     if (!folded && (rc = lex3_fold(ctx, r))) return rc;
-    CK(cudaFuncSetAttribute(lex3_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->l3_walk_smem));
-    CK(cudaFuncSetAttribute(lex3_walk_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     if ((rc = lex3_grid(ctx, r, (const void*)lex3_walk_kernel, LX_THREADS, ctx->l3_walk_smem, r.wide, &g3)))
         return rc;
     if ((rc = lex3_scan(ctx, r))) return rc;
@@ -831,10 +886,8 @@ int lex3_front(alp_ctx* ctx, Lex3Run& r, bool folded = false) {
 // exclusive (count, last start) over the tiles
 int lex3_tiles(alp_ctx* ctx, Lex3Run& r) {
     const long long lchunks = (r.tiles + LT_CHUNK - 1) / LT_CHUNK;
-    unsigned long long* ccs = reinterpret_cast<unsigned long long*>(r.base + r.o_ccs);
-    lex3_tile_reduce_kernel<<<(unsigned)lchunks, LT_CHUNK, 0, ctx->stream>>>(r.a.tile_cs, r.tiles, ccs);
-    CK(cudaGetLastError());
-    lex3_tile_scan_kernel<<<(unsigned)lchunks, LT_CHUNK, 0, ctx->stream>>>(r.a.tile_cs, r.tiles, ccs, r.a.res);
+    lex3_tile_scan_kernel<<<(unsigned)lchunks, LT_CHUNK, 0, ctx->stream>>>(r.a.tile_cs, r.tiles, r.lex_sync,
+                                                                           r.sg.sentinels ? 2 * r.nd : 0, r.a.res);
     CK(cudaGetLastError());
     return ALP_OK;
 }
@@ -845,13 +898,11 @@ int lex3_emit(alp_ctx* ctx, Lex3Run& r, bool tiles_done = false) {
     const size_t sm = r.walked ? lex3_write_smem() : ctx->l3_emit_smem;
     unsigned g5;
     int rc;
-    CK(cudaFuncSetAttribute(k5, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    CK(cudaFuncSetAttribute(k5, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     if ((rc = lex3_grid(ctx, r, k5, LX_THREADS, sm, r.walked ? r.wide : r.tiles, &g5))) return rc;
     mark(ctx, "start");
     if (!tiles_done) {
         if ((rc = lex3_tiles(ctx, r))) return rc;
-        mark(ctx, "lex3_tile_reduce+lex3_tile_scan");
+        mark(ctx, "lex3_tile_scan_kernel");
     }
     {
         void* args[] = {&r.a, &r.sg};
@@ -884,8 +935,6 @@ int lex3_tok(alp_ctx* ctx, Lex3Run& r, long long* total) {
     unsigned g;
     int rc;
     const size_t sm = lex3_tok_smem(ctx->S);
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     if ((rc = lex3_grid(ctx, r, (const void*)k, LX_THREADS, sm, r.tiles, &g))) return rc;
     CK(cudaMemsetAsync(r.a.tile_cs, 0, 8 * (size_t)r.tiles, ctx->stream));  // look-back words
     mark(ctx, "start");
@@ -913,8 +962,7 @@ int lex3_scan(alp_ctx* ctx, Lex3Run& r) {
     const void* k = scan_kernel_for(scan_g(ctx));
     unsigned g2;
     int rc;
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->l3_scan_smem));
-    if ((rc = lex3_grid(ctx, r, k, LS_WARPS * 32, ctx->l3_scan_smem, r.stiles, &g2))) return rc;
+    if ((rc = lex3_grid(ctx, r, k, LS_WARPS * 32, ctx->l3_scan_smem, r.stiles, &g2, false))) return rc;
     mark(ctx, "start");
     {
         void* args[] = {&r.a};
@@ -953,7 +1001,7 @@ int lex3_run_alloc(alp_ctx* ctx, const uint8_t* d_in, long long n, const long lo
         return rc;
     mark(ctx, "start");
     if ((rc = lex3_tiles(ctx, r))) return rc;
-    mark(ctx, "lex3_tile_reduce+lex3_tile_scan");
+    mark(ctx, "lex3_tile_scan_kernel");
     CK(cudaMemcpyAsync(ctx->h_res, r.a.res, sizeof(AlpResult), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (ctx->h_res->error & ALP_DEV_ERR_TIMEOUT) return fail(ctx, ALP_ERR_TIMEOUT, "lexer look-back timed out");
@@ -1059,10 +1107,6 @@ int put_doc_off(alp_ctx* ctx, long long n) {
     return ALP_OK;
 }
 
-// Positions (⊢ tokens ⊣ per document, L of them) already in
-// tmp[T_TTERM..T_TEND] and per-document validity in `dvalid` -> tree.
-// `want_tree` 0 gives the production sequence only.  Node offsets of the
-// documents land in tmp[T_NODEOFF].
 // Output buffers for N nodes (context-owned when ctx_out) and the node and
 // bracket intermediates for N nodes and K kept brackets.
 // `exact`: N is the node count, for which a caller's allocator can be asked.  `general`:
@@ -1104,6 +1148,47 @@ int parse_buffers(alp_ctx* ctx, ParseOut* o, int ctx_out, long long N, long long
     return ALP_OK;
 }
 
+// Pair ids and scanned tile sums of the positions of `a` (a.dL: a.L is a capacity).  sy: the
+// scan's ticket and flags, cleared; its chunk sums lie after the tile sums.
+int position_sums(alp_ctx* ctx, ParseArgs& a, ScanSync sy, long long nd) {
+    const long long tiles = (a.L + PP_TILE - 1) / PP_TILE, chunks = (tiles + ST_CHUNK - 1) / ST_CHUNK;
+    int rc, per1 = 0;
+    if ((rc = grow(ctx, ctx->tmp[T_PID], (size_t)a.L * 2 + 64)) ||
+        (rc = grow(ctx, ctx->tmp[T_TSUMS], (size_t)(tiles + chunks + 1) * sizeof(PosSums))))
+        return rc;
+    a.pid = (uint16_t*)ctx->tmp[T_PID].p;
+    a.tile_sums = (PosSums*)ctx->tmp[T_TSUMS].p;
+    sy.sums = a.tile_sums + tiles;
+    const void* fn = pairs_kernel_for(ctx->pt.q, ctx->pt.k);
+    const size_t sm = pairs_smem_bytes(ctx->pt.n_pairs, ctx->pt.q + ctx->pt.k);
+    if ((rc = fit_blocks(ctx, fn, PP_THREADS, sm, false, &per1))) return rc;
+    const long long x = (long long)persistent_ctas(per1, ctx->tune.pairs_ctas) * ctx->sms;
+    mark(ctx, "start");
+    {
+        void* args[] = {&a};
+        CK(cudaLaunchKernel(fn, dim3((unsigned)(x < tiles ? x : tiles)), dim3(PP_THREADS), args, sm, ctx->stream));
+    }
+    mark(ctx, "parse_pairs_kernel");
+    scan_tiles_kernel<<<(unsigned)chunks, ST_CHUNK, 0, ctx->stream>>>(a.tile_sums, tiles, sy, a.res, a.node_off, a.br_off,
+                                                                     nd, a.dL);
+    CK(cudaGetLastError());
+    mark(ctx, "scan_tiles_kernel");
+    return ALP_OK;
+}
+
+// The parser's result and the position scan's words alone at the head of the scratch, for
+// positions that no lexer run of this call put there.
+int positions_head(alp_ctx* ctx, long long L, AlpResult** res, ScanSync* sy) {
+    const size_t chunks = (size_t)L / ((size_t)PP_TILE * ST_CHUNK) + 2;
+    int rc;
+    if ((rc = grow(ctx, ctx->scratch, SC_COPY + 4 * chunks))) return rc;
+    uint8_t* base = reinterpret_cast<uint8_t*>(ctx->scratch.p);
+    CK(cudaMemsetAsync(base, 0, SC_COPY + 4 * chunks, ctx->stream));
+    *res = reinterpret_cast<AlpResult*>(base);
+    *sy = ScanSync{reinterpret_cast<unsigned int*>(base + SC_TICKETS) + TK_POS_TILES, reinterpret_cast<uint32_t*>(base + SC_COPY), nullptr};
+    return ALP_OK;
+}
+
 // The expand kernel with the pair lookup and a look-back over tiles in it,
 // for a grammar's (q, k) (see parse_pairs_kernel).
 inline const void* fused_expand_for(int q, int k) {
@@ -1121,34 +1206,36 @@ inline const void* fused_expand_for(int q, int k) {
 int expand_smem(alp_ctx* ctx, const void* fn, size_t base, int* span_cap, size_t* sm) {
     *sm = base;
     *span_cap = 0;
-    int fit = 0, per_sm = 0, reserved = 0, optin = 0;
-    cudaFuncAttributes fa;
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)base));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, PP_THREADS, base));
-    CK(cudaFuncGetAttributes(&fa, fn));
-    CK(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device));
-    CK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, ctx->device));
-    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    int rc, fit = 0;
+    if ((rc = fit_blocks(ctx, fn, PP_THREADS, base, false, &fit))) return rc;
     const int ctas = persistent_ctas(fit, ctx->tune.expand_ctas);
-    long long room = (long long)per_sm / ctas - reserved - (long long)fa.sharedSizeBytes - (long long)base;
-    room = std::min(room, (long long)optin - (long long)fa.sharedSizeBytes - (long long)base);
+    for (const alp_ctx::SpanFit& f : ctx->span_fits)
+        if (f.fn == fn && f.base == base && f.ctas == ctas) {
+            *sm = f.sm;
+            *span_cap = f.span_cap;
+            return ALP_OK;
+        }
+    cudaFuncAttributes fa;
+    CK(cudaFuncGetAttributes(&fa, fn));
+    long long room = (long long)ctx->sm_smem / ctas - ctx->sm_reserved - (long long)fa.sharedSizeBytes - (long long)base;
+    room = std::min(room, (long long)ctx->sm_optin - (long long)fa.sharedSizeBytes - (long long)base);
     room = std::min(room, (long long)EX_SPAN_BYTES) & ~31LL;
-    if (room < 1024) return ALP_OK;
-    int fit2 = 0;
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(base + room)));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit2, fn, PP_THREADS, base + room));
-    if (fit2 < ctas) return ALP_OK;  // token spans through L1, as without the stage
-    *span_cap = (int)(room / 8);      // a multiple of 4
-    *sm = base + (size_t)room;
+    if (room >= 1024) {
+        int fit2 = 0;
+        if ((rc = fit_blocks(ctx, fn, PP_THREADS, base + (size_t)room, false, &fit2))) return rc;
+        if (fit2 >= ctas) {  // else token spans through L1
+            *span_cap = (int)(room / 8);  // a multiple of 4
+            *sm = base + (size_t)room;
+        }
+    }
+    ctx->span_fits.push_back({fn, base, *sm, ctas, *span_cap});
     return ALP_OK;
 }
 
 int expand_grid(alp_ctx* ctx, const void* fn, size_t sm2, long long tiles, unsigned* g) {
-    int sms = 0, per2 = 0;
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, fn, PP_THREADS, sm2));
-    const long long x = (long long)persistent_ctas(per2, ctx->tune.expand_ctas) * sms;
+    int rc, per2 = 0;
+    if ((rc = fit_blocks(ctx, fn, PP_THREADS, sm2, false, &per2))) return rc;
+    const long long x = (long long)persistent_ctas(per2, ctx->tune.expand_ctas) * ctx->sms;
     *g = (unsigned)(x < tiles ? x : tiles);
     return ALP_OK;
 }
@@ -1222,12 +1309,108 @@ int run_tree(alp_ctx* ctx, TreeArgs& t, bool one) {
 int run_tree_escapes(alp_ctx* ctx, TreeArgs& t) {
     const long long tiles = (t.L + PP_TILE - 1) / PP_TILE;
     mark(ctx, "start");
-    tree_levels_kernel<<<(unsigned)(((tiles + 31) / 32 + 255) / 256), 256, 0, ctx->stream>>>(t, tiles);
-    CK(cudaGetLastError());
+    if (tiles > 32) {  // else the tiles' own minima are one group: no search goes above them
+        tree_levels_kernel<<<(unsigned)(((tiles + 31) / 32 + 255) / 256), 256, 0, ctx->stream>>>(t, tiles);
+        CK(cudaGetLastError());
+    }
     const long long g = (tiles + 7) / 8;
     tree_escape_kernel<<<(unsigned)(g < 148 * 8 ? g : 148 * 8), 256, 0, ctx->stream>>>(t, tiles);
     CK(cudaGetLastError());
     mark(ctx, "tree_levels+tree_escape");
+    return ALP_OK;
+}
+
+// A parse whose positions and parser results share one cleared head of the scratch (SC_*):
+// `a` is filled in; `summed`: its pair ids and tile sums are there and their result read.
+struct PosHead {
+    uint8_t* base = nullptr;
+    ScanSync sy{};
+    ParseArgs a{};
+    bool summed = false;
+    bool ids = false;  // token ids from the caller: the head's first result says if one was refused
+};
+
+AlpResult* head_result(const PosHead& h) { return reinterpret_cast<AlpResult*>(h.base + SC_PARSE); }
+
+// The head in one copy and wait: the parser's result to ctx->h_res, the first result to *lex.
+int read_head(alp_ctx* ctx, const PosHead& h, AlpResult* lex, uint8_t* valid) {
+    CK(cudaMemcpyAsync(ctx->h_res, h.base, SC_COPY, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    CK(cudaGetLastError());
+    const uint8_t* c = reinterpret_cast<const uint8_t*>(ctx->h_res);
+    if (lex) memcpy(lex, c, sizeof *lex);
+    if (valid) *valid = c[SC_VALID];
+    AlpResult pr;
+    memcpy(&pr, c + SC_PARSE, sizeof pr);
+    *ctx->h_res = pr;
+    return ALP_OK;
+}
+
+int result_error(alp_ctx* ctx) {
+    if (ctx->h_res->error & ALP_DEV_ERR_TIMEOUT) return fail(ctx, ALP_ERR_TIMEOUT, "kernel wait timed out");
+    if (ctx->h_res->error & ALP_DEV_ERR_CAPACITY) return fail(ctx, ALP_ERR_CAPACITY, "internal buffer too small");
+    return ALP_OK;
+}
+
+// What every form of the position pass reads and writes, for L positions in
+// tmp[T_TTERM..T_TEND].
+int parse_args(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, int want_tree, AlpResult* d_res, ParseArgs& a) {
+    int rc;
+    if ((rc = grow(ctx, ctx->tmp[T_NODEOFF], (size_t)(nd + 1) * 8)) || (rc = grow(ctx, ctx->tmp[T_BROFF], (size_t)(nd + 1) * 8)))
+        return rc;
+    memset(&a, 0, sizeof a);
+    a.t = ctx->pt;
+    a.P = (const uint16_t*)ctx->tmp[T_TTERM].p;
+    a.pstart = (const uint32_t*)ctx->tmp[T_TSTART].p;
+    a.pend = (const uint32_t*)ctx->tmp[T_TEND].p;
+    a.L = L;
+    a.n_docs = nd;
+    a.res = d_res;
+    a.node_off = (long long*)ctx->tmp[T_NODEOFF].p;
+    a.br_off = (long long*)ctx->tmp[T_BROFF].p;
+    a.doc_valid = dvalid;
+    a.subst_terminals = want_tree;
+    return ALP_OK;
+}
+
+// Inputs of at most this many positions go from the lexer to the pair sums without a host
+// wait in between: the position count stays on the device and the pair ids are sized for the
+// capacity.  With the tile scans of one launch each and the launch limits asked once, a call
+// went from 161 to 125 us at 1 KB, 207 to 168 at 1 MB and 215 to 171 at 4 MB.  A wait is some
+// 15 us of whatever the call takes, 3 % of it at 16 Mi positions, where the ids' capacity (2 B
+// a byte of input against 0.6 at the exact count) starts to count instead.
+constexpr long long AHEAD_MAX = 1ll << 24;
+
+bool ahead_ok(const alp_ctx* ctx, long long n, long long nd) {
+    return ctx->lex3 && ctx->tune.lex_split && ctx->tune.parse_split && n > 0 && n + 2 * nd <= AHEAD_MAX;
+}
+
+// Lexer and pair sums of n bytes in one run of launches, with one wait for both results.
+// *m: tokens.  valid (one document): the lexer's verdict, and *dvalid moves into the head.
+int lex_pairs(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long* d_off, long long nd, long long tcap,
+              uint8_t** dvalid, PosHead* h, long long* m, uint8_t* valid) {
+    Lex3Run r;
+    int rc;
+    if ((rc = grow(ctx, ctx->tmp[T_TOKOFF], (size_t)(nd + 1) * 8)) ||
+        (rc = lex3_prepare(ctx, d_in, n, d_off, nd, 1, ctx->tmp[T_TTERM].p, ctx->tmp[T_TSTART].p, ctx->tmp[T_TEND].p, tcap,
+                           *dvalid, r)))
+        return rc;
+    if (valid) r.sg.valid = *dvalid = r.base + SC_VALID;
+    h->base = r.base;
+    h->sy = r.pos_sync;
+    if ((rc = lex3_front(ctx, r)) || (rc = lex3_emit<uint16_t, uint32_t>(ctx, r)) ||
+        (rc = parse_args(ctx, n + 2 * nd, nd, *dvalid, 1, head_result(*h), h->a)))
+        return rc;
+    h->a.dL = &r.a.res->aux[5];
+    AlpResult lex;
+    if ((rc = position_sums(ctx, h->a, h->sy, nd)) || (rc = read_head(ctx, *h, &lex, valid))) return rc;
+    if (lex.error & ALP_DEV_ERR_TIMEOUT) return fail(ctx, ALP_ERR_TIMEOUT, "lexer look-back timed out");
+    ctx->last_tokens = *m = lex.count;
+    if (lex.error & ALP_DEV_ERR_CAPACITY) return fail(ctx, ALP_ERR_CAPACITY, "token buffer too small");
+    if (lex.aux[5] != lex.count + 2 * nd) return fail(ctx, ALP_ERR_CUDA, "token counts disagree");
+    h->a.dL = nullptr;
+    h->a.L = lex.aux[5];
+    h->summed = true;
     return ALP_OK;
 }
 
@@ -1243,31 +1426,25 @@ int run_tree_escapes(alp_ctx* ctx, TreeArgs& t) {
 // again at the exact sizes it reported.  The first parse on a context, and
 // grammars whose counts could pass 32 bits, take the two-pass form: the pair
 // kernel and a scan of its tile sums give the exact sizes first.
-// h_valid0 (pinned, optional): document 0's validity, read in the same final wait.
+// valid0 (optional): document 0's validity, read in the same final wait.  head: the head of
+// this call when a lexer run or the caller's tokens set it up, with dvalid in it for one document.
 int parse_positions(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, ParseOut* o, int64_t cap, int ctx_out,
-                    int64_t* n_node, int want_tree, uint8_t* h_valid0 = nullptr) {
+                    int64_t* n_node, int want_tree, uint8_t* valid0 = nullptr, PosHead* head = nullptr) {
     *n_node = 0;
     if (L >= 0x7fffffffLL) return fail(ctx, ALP_ERR_ARG, "too many positions (%lld)", L);
     const long long tiles = (L + PP_TILE - 1) / PP_TILE;
     int rc;
-    if ((rc = grow(ctx, ctx->tmp[T_NODEOFF], (size_t)(nd + 1) * 8)) || (rc = grow(ctx, ctx->tmp[T_BROFF], (size_t)(nd + 1) * 8)) ||
-        (rc = grow(ctx, ctx->scratch, 256)))
-        return rc;
-    AlpResult* d_res = reinterpret_cast<AlpResult*>(ctx->scratch.p);
-    if ((rc = set_result(ctx, d_res, 1))) return rc;
+    AlpResult* d_res;
+    ScanSync sy;
     ParseArgs a;
-    memset(&a, 0, sizeof a);
-    a.t = ctx->pt;
-    a.P = (const uint16_t*)ctx->tmp[T_TTERM].p;
-    a.pstart = (const uint32_t*)ctx->tmp[T_TSTART].p;
-    a.pend = (const uint32_t*)ctx->tmp[T_TEND].p;
-    a.L = L;
-    a.n_docs = nd;
-    a.res = d_res;
-    a.node_off = (long long*)ctx->tmp[T_NODEOFF].p;
-    a.br_off = (long long*)ctx->tmp[T_BROFF].p;
-    a.doc_valid = dvalid;
-    a.subst_terminals = want_tree;
+    if (head) {
+        d_res = head_result(*head);
+        sy = head->sy;
+    } else if ((rc = positions_head(ctx, L, &d_res, &sy))) {
+        return rc;
+    }
+    if (head && head->summed) a = head->a;
+    else if ((rc = parse_args(ctx, L, nd, dvalid, want_tree, d_res, a))) return rc;
     if (expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack) > 220 * 1024)
         return fail(ctx, ALP_ERR_TABLE, "parser tables too large for shared memory");
     size_t sm2 = expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack);
@@ -1316,39 +1493,17 @@ int parse_positions(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, Pa
         a.cap_brs = K;
     } else {
         // ---- two passes: pair ids and tile sums, their scan, the sizes, then expand
-        if ((rc = grow(ctx, ctx->tmp[T_PID], (size_t)L * 2 + 64)) ||
-            (rc = grow(ctx, ctx->tmp[T_TSUMS], (tiles + tiles / ST_CHUNK + 2) * sizeof(PosSums))))
-            return rc;
-        a.pid = (uint16_t*)ctx->tmp[T_PID].p;
-        a.tile_sums = (PosSums*)ctx->tmp[T_TSUMS].p;
-        const size_t sm1 = pairs_smem_bytes(ctx->pt.n_pairs, ctx->pt.q + ctx->pt.k);
-        CK(cudaFuncSetAttribute(pairs_kernel_for(ctx->pt.q, ctx->pt.k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
-        mark(ctx, "start");
-        unsigned g_pairs = 1, g_expand = 1;
-        {
-            int sms = 0, per1 = 0;
-            CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, pairs_kernel_for(ctx->pt.q, ctx->pt.k), PP_THREADS, sm1));
-            const long long x = (long long)persistent_ctas(per1, ctx->tune.pairs_ctas) * sms;
-            g_pairs = (unsigned)(x < tiles ? x : tiles);
+        unsigned g_expand = 1;
+        AlpResult ids{};
+        if (!head) {
+            if ((rc = position_sums(ctx, a, sy, nd)) || (rc = read_result(ctx, d_res))) return rc;
+        } else {
+            if (!head->summed &&
+                ((rc = position_sums(ctx, a, sy, nd)) || (rc = read_head(ctx, *head, &ids, nullptr))))
+                return rc;
+            if (head->ids && ids.aux[0]) return fail(ctx, ALP_ERR_ARG, "terminal id out of range");
+            if ((rc = result_error(ctx))) return rc;
         }
-        {
-            void* args[] = {&a};
-            CK(cudaLaunchKernel(pairs_kernel_for(ctx->pt.q, ctx->pt.k), dim3(g_pairs), dim3(PP_THREADS), args, sm1,
-                                ctx->stream));
-        }
-        mark(ctx, "parse_pairs_kernel");
-        {
-            const long long chunks = (tiles + ST_CHUNK - 1) / ST_CHUNK;
-            PosSums* csum = a.tile_sums + tiles;  // chunk sums after the tile sums
-            scan_tiles_reduce_kernel<<<(unsigned)chunks, ST_CHUNK, 0, ctx->stream>>>(a.tile_sums, tiles, csum, nullptr);
-            CK(cudaGetLastError());
-            scan_tiles_kernel<<<(unsigned)chunks, ST_CHUNK, 0, ctx->stream>>>(a.tile_sums, tiles, csum, d_res, a.node_off,
-                                                                             a.br_off, nd, nullptr);
-            CK(cudaGetLastError());
-        }
-        mark(ctx, "scan_tiles_reduce+scan_tiles");
-        if ((rc = read_result(ctx, d_res))) return rc;
         // nodes, brackets, and brackets left after closing adjacent pairs
         N = ctx->h_res->aux[0];
         B = ctx->h_res->aux[1];
@@ -1432,7 +1587,6 @@ int parse_positions(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, Pa
         }
         if ((rc = run_ple(ctx, a.dsbuf, K, a.brbuf, nullptr, T_B_TMIN, a.br_off, nd, dvalid, d_res))) return rc;
     }
-    if (h_valid0) CK(cudaMemcpyAsync(h_valid0, dvalid, 1, cudaMemcpyDeviceToHost, ctx->stream));
     if (fused && ctx_out && ctx->alloc_fn) {
         // written at estimated capacities: copied into the allocator's buffers
         void* p[5] = {};
@@ -1444,7 +1598,15 @@ int parse_positions(alp_ctx* ctx, long long L, long long nd, uint8_t* dvalid, Pa
         *o = ParseOut{(int64_t*)p[0], (uint32_t*)p[1], (uint8_t*)p[2], (int64_t*)p[3], (int64_t*)p[4]};
     }
     if (ctx_out && (rc = batch_out(ctx, a.node_off, dvalid, nd))) return rc;
-    if ((rc = read_result(ctx, d_res))) return rc;
+    if (head) {
+        AlpResult ids{};
+        if ((rc = read_head(ctx, *head, &ids, valid0)) || (rc = result_error(ctx))) return rc;
+        if (head->ids && ids.aux[1] && valid0) *valid0 = 0;  // a token of no terminal
+    } else {
+        if (valid0) CK(cudaMemcpyAsync(ctx->h_stage, dvalid, 1, cudaMemcpyDeviceToHost, ctx->stream));
+        if ((rc = read_result(ctx, d_res))) return rc;
+        if (valid0) memcpy(valid0, ctx->h_stage, 1);
+    }
     *n_node = N;
     return ALP_OK;
 }
@@ -1472,10 +1634,10 @@ int lex_core(alp_ctx* ctx, const uint8_t* d_in, int64_t n, TermT* term, PosT* st
     }
     if (ctx->lex3 && !ctx->state_out) {
         int rc;
-        if ((rc = grow(ctx, ctx->tmp[T_DVALID], 16)) || (rc = put_doc_off(ctx, n))) return rc;
+        if ((rc = grow(ctx, ctx->tmp[T_DVALID], 16))) return rc;
         uint8_t* dvalid = (uint8_t*)ctx->tmp[T_DVALID].p;
         long long total = 0;
-        rc = lex_seg<TermT, PosT>(ctx, d_in, n, (const long long*)ctx->tmp[T_DOCOFF].p, 1, 0, term, start, end, cap,
+        rc = lex_seg<TermT, PosT>(ctx, d_in, n, nullptr, 1, 0, term, start, end, cap,
                                   dvalid, &total);
         *count = total;
         if (rc) return rc;
@@ -1503,34 +1665,44 @@ int parse_core(alp_ctx* ctx, const uint8_t* d_in, int64_t n, ParseOut* o, int64_
     int rc;
     const size_t tcap = (size_t)n + 2 + 16;
     if ((rc = grow(ctx, ctx->tmp[T_TTERM], tcap * 2)) || (rc = grow(ctx, ctx->tmp[T_TSTART], tcap * 4)) ||
-        (rc = grow(ctx, ctx->tmp[T_TEND], tcap * 4)) || (rc = grow(ctx, ctx->tmp[T_DVALID], 16)) ||
-        (rc = put_doc_off(ctx, n)))
+        (rc = grow(ctx, ctx->tmp[T_TEND], tcap * 4)) || (rc = grow(ctx, ctx->tmp[T_DVALID], 16)))
         return rc;
     uint8_t* dvalid = (uint8_t*)ctx->tmp[T_DVALID].p;
     long long m = 0;
-    // the document's validity comes back with the lexer's token count and with the
-    // parser's final counts (pinned bytes in h_stage), not in waits of their own
-    uint8_t* hv = reinterpret_cast<uint8_t*>(ctx->h_stage) + 200;
-    hv[0] = 0;  // stays 0 for an empty input (the lexer then launches nothing)
-    hv[1] = 0;
-    ctx->lex_valid0 = hv;
-    rc = lex_seg<uint16_t, uint32_t>(ctx, d_in, n, (const long long*)ctx->tmp[T_DOCOFF].p, 1, 1,
-                                     (uint16_t*)ctx->tmp[T_TTERM].p, (uint32_t*)ctx->tmp[T_TSTART].p,
-                                     (uint32_t*)ctx->tmp[T_TEND].p, (long long)tcap, dvalid, &m);
-    ctx->lex_valid0 = nullptr;
-    if (rc) return rc;
-    if (!hv[0]) return ALP_OK;
+    uint8_t v = 0;
+    PosHead head;
+    const bool ahead = ahead_ok(ctx, n, 1);
+    if (ahead) {
+        if ((rc = lex_pairs(ctx, d_in, n, nullptr, 1, (long long)tcap, &dvalid, &head, &m, &v))) return rc;
+        if (!v) return ALP_OK;
+    } else {
+        // the document's validity comes back with the lexer's token count, not in a wait of its own
+        uint8_t* hv = reinterpret_cast<uint8_t*>(ctx->h_stage) + 200;
+        hv[0] = 0;  // stays 0 for an empty input (the lexer then launches nothing)
+        if (!ctx->lex3 && (rc = put_doc_off(ctx, n))) return rc;
+        ctx->lex_valid0 = hv;
+        rc = lex_seg<uint16_t, uint32_t>(ctx, d_in, n, ctx->lex3 ? nullptr : (const long long*)ctx->tmp[T_DOCOFF].p, 1, 1,
+                                         (uint16_t*)ctx->tmp[T_TTERM].p, (uint32_t*)ctx->tmp[T_TSTART].p,
+                                         (uint32_t*)ctx->tmp[T_TEND].p, (long long)tcap, dvalid, &m);
+        ctx->lex_valid0 = nullptr;
+        if (rc) return rc;
+        if (!hv[0]) return ALP_OK;
+    }
     int64_t N = 0;
-    rc = parse_positions(ctx, m + 2, 1, dvalid, o, cap, ctx_out, &N, 1, hv + 1);
+    rc = parse_positions(ctx, m + 2, 1, dvalid, o, cap, ctx_out, &N, 1, &v, ahead ? &head : nullptr);
     if (rc) { *n_node = N; return rc; }
-    *valid = hv[1] ? 1 : 0;
+    *valid = v ? 1 : 0;
     *n_node = *valid ? N : 0;
     return ALP_OK;
 }
 
 // Token arrays from the caller (uint32 ids, int64 spans) -> positions ⊢ tokens ⊣.
+// res->aux[0]: an id past 16 bits or a sentinel's (an error); aux[1]: an id of no terminal (the
+// tokens are then no sentence; the position takes `filler`, so that no key leaves the table).
 __global__ void tokens_in_kernel(const uint32_t* term, const int64_t* ts, const int64_t* te, long long m, uint16_t* P,
-                                 uint32_t* s32, uint32_t* e32, uint32_t sl, uint32_t sr, AlpResult* res) {
+                                 uint32_t* s32, uint32_t* e32, uint32_t sl, uint32_t sr, uint32_t T, uint32_t filler,
+                                 AlpResult* res, uint8_t* valid) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *valid = 1;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m + 2; i += (long long)gridDim.x * blockDim.x) {
         if (i == 0 || i == m + 1) {
             P[i] = (uint16_t)(i == 0 ? sl : sr);
@@ -1538,29 +1710,38 @@ __global__ void tokens_in_kernel(const uint32_t* term, const int64_t* ts, const 
             e32[i] = 0;
             continue;
         }
-        const uint32_t t = term[i - 1];
-        if (t > 0xffffu || t == sl || t == sr) res->valid = 0;
+        uint32_t t = term[i - 1];
+        if (t > 0xffffu || t == sl || t == sr) res->aux[0] = 1;
+        if (t >= T) {
+            res->aux[1] = 1;
+            t = filler;
+        }
         P[i] = (uint16_t)t;
         s32[i] = ts ? (uint32_t)ts[i - 1] : 0u;
         e32[i] = te ? (uint32_t)te[i - 1] : 0u;
     }
 }
 
-int tokens_in(alp_ctx* ctx, const uint32_t* term, const int64_t* ts, const int64_t* te, int64_t m) {
+// The caller's m tokens as positions, their validity and the parser's head in the scratch.
+// A refused id is seen with the pair sums' result, or here before the fused position pass.
+int tokens_in(alp_ctx* ctx, const uint32_t* term, const int64_t* ts, const int64_t* te, int64_t m, PosHead* h) {
     int rc;
+    AlpResult* lex;
     if ((rc = grow(ctx, ctx->tmp[T_TTERM], (size_t)(m + 2) * 2 + 16)) || (rc = grow(ctx, ctx->tmp[T_TSTART], (size_t)(m + 2) * 4 + 16)) ||
-        (rc = grow(ctx, ctx->tmp[T_TEND], (size_t)(m + 2) * 4 + 16)) || (rc = grow(ctx, ctx->scratch, 256)) ||
-        (rc = grow(ctx, ctx->tmp[T_DVALID], 16)))
+        (rc = grow(ctx, ctx->tmp[T_TEND], (size_t)(m + 2) * 4 + 16)) || (rc = positions_head(ctx, m + 2, &lex, &h->sy)))
         return rc;
-    AlpResult* d_res = reinterpret_cast<AlpResult*>(ctx->scratch.p);
-    if ((rc = set_result(ctx, d_res, 1))) return rc;
-    tokens_in_kernel<<<148 * 4, 256, 0, ctx->stream>>>(term, ts, te, m, (uint16_t*)ctx->tmp[T_TTERM].p,
-                                                      (uint32_t*)ctx->tmp[T_TSTART].p, (uint32_t*)ctx->tmp[T_TEND].p,
-                                                      ctx->pt.start, ctx->pt.end, d_res);
+    h->base = reinterpret_cast<uint8_t*>(lex);
+    h->ids = true;
+    const long long g = (m + 2 + 255) / 256;
+    tokens_in_kernel<<<(unsigned)(g < 148 * 8 ? g : 148 * 8), 256, 0, ctx->stream>>>(
+        term, ts, te, m, (uint16_t*)ctx->tmp[T_TTERM].p, (uint32_t*)ctx->tmp[T_TSTART].p, (uint32_t*)ctx->tmp[T_TEND].p,
+        ctx->pt.start, ctx->pt.end, (uint32_t)ctx->pt.T, ctx->pt.empty, lex, h->base + SC_VALID);
     CK(cudaGetLastError());
-    if ((rc = read_result(ctx, d_res))) return rc;
-    if (!ctx->h_res->valid) return fail(ctx, ALP_ERR_ARG, "terminal id out of range");
-    CK(cudaMemsetAsync(ctx->tmp[T_DVALID].p, 1, 1, ctx->stream));
+    if (!ctx->tune.parse_split) {
+        AlpResult ids;
+        if ((rc = read_head(ctx, *h, &ids, nullptr))) return rc;
+        if (ids.aux[0]) return fail(ctx, ALP_ERR_ARG, "terminal id out of range");
+    }
     return ALP_OK;
 }
 
@@ -1706,6 +1887,12 @@ int parse_batch_core(alp_ctx* ctx, const uint8_t* d_in, const int64_t* d_off, in
         return rc;
     uint8_t* dvalid = (uint8_t*)ctx->tmp[T_DVALID].p;
     long long m = 0;
+    if (ahead_ok(ctx, n, n_docs)) {
+        PosHead head;
+        if ((rc = lex_pairs(ctx, d_in, n, (const long long*)d_off, n_docs, (long long)tcap, &dvalid, &head, &m, nullptr)))
+            return rc;
+        return parse_positions(ctx, m + 2 * n_docs, n_docs, dvalid, o, 0, 1, N, 1, nullptr, &head);
+    }
     rc = lex_seg<uint16_t, uint32_t>(ctx, d_in, n, (const long long*)d_off, n_docs, 1, (uint16_t*)ctx->tmp[T_TTERM].p,
                                      (uint32_t*)ctx->tmp[T_TSTART].p, (uint32_t*)ctx->tmp[T_TEND].p, (long long)tcap,
                                      dvalid, &m);
@@ -1747,7 +1934,7 @@ int alp_ctx_create(const void* blob, size_t len, int device, alp_ctx** out) {
         if (!rc && (ctx->pt.start >= T || ctx->pt.end >= T || ctx->pt.empty >= T))
             rc = fail(ctx, ALP_ERR_TABLE, "parser sentinel ids out of range");
     }
-    if (!rc && cudaMallocHost(&ctx->h_res, sizeof(AlpResult)) != cudaSuccess)
+    if (!rc && cudaMallocHost(&ctx->h_res, SC_COPY) != cudaSuccess)
         rc = fail(ctx, ALP_ERR_CUDA, "cudaMallocHost failed");
     if (!rc && cudaMallocHost(&ctx->h_stage, 256) != cudaSuccess) rc = fail(ctx, ALP_ERR_CUDA, "cudaMallocHost failed");
     if (rc) {
@@ -1992,10 +2179,9 @@ int alp_tune_parse(alp_ctx* ctx, const uint8_t* d_in, int64_t n, int reps, char*
         const size_t sm2 = expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack);
         const void* ex = ctx->tune.parse_split ? (const void*)parse_expand_kernel<0, 0, false>
                                                : fused_expand_for(ctx->pt.q, ctx->pt.k);
-        CK(cudaFuncSetAttribute(pairs_kernel_for(ctx->pt.q, ctx->pt.k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
-        CK(cudaFuncSetAttribute(ex, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit_pairs, pairs_kernel_for(ctx->pt.q, ctx->pt.k), PP_THREADS, sm1));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit_expand, ex, PP_THREADS, sm2));
+        if ((rc = fit_blocks(ctx, pairs_kernel_for(ctx->pt.q, ctx->pt.k), PP_THREADS, sm1, false, &fit_pairs)) ||
+            (rc = fit_blocks(ctx, ex, PP_THREADS, sm2, false, &fit_expand)))
+            return done(rc);
     }
     best = 1e30;
     arg = 0;
@@ -2331,9 +2517,7 @@ int alp_lex(alp_ctx* ctx, const uint8_t* d_in, int64_t n, uint32_t** d_term, int
         *n_tok = 0;
         *valid = 0;
         if ((rc = grow(ctx, ctx->tmp[T_DVALID], 16)) || (rc = grow(ctx, ctx->tmp[T_TOKOFF], 16)) ||
-            (rc = put_doc_off(ctx, n)) ||
-            (rc = lex3_run_alloc(ctx, d_in, n, (const long long*)ctx->tmp[T_DOCOFF].p, 1,
-                                 (uint8_t*)ctx->tmp[T_DVALID].p, p, &total, valid)))
+            (rc = lex3_run_alloc(ctx, d_in, n, nullptr, 1, (uint8_t*)ctx->tmp[T_DVALID].p, p, &total, valid)))
             return rc;
         *n_tok = total;
         *d_term = (uint32_t*)p[0];
@@ -2766,7 +2950,7 @@ int alp_lex_shard_count(alp_lex_shard* s, uint32_t entry_state, int64_t* n_tok, 
     if ((rc = lex3_front(ctx, s->r, true)) || (rc = lex3_tiles(ctx, s->r))) return rc;
     lex3_shard_totals_kernel<<<1, LX_THREADS, 0, ctx->stream>>>(s->r.a, s->d_tot);
     CK(cudaGetLastError());
-    mark(ctx, "lex3_tile_reduce+lex3_tile_scan+lex3_shard_totals_kernel");
+    mark(ctx, "lex3_tile_scan+lex3_shard_totals");
     CK(cudaMemcpyAsync(s->h, s->d_tot, 16, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(s->h + 2, &s->r.a.res->error, 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -2991,36 +3175,17 @@ int alp_parse_shard_sums(alp_parse_shard* s, const uint32_t* halo_l, const uint3
     };
     s->prev_pair = s->first ? NO_PAIR : host_pair(ctx->ph, at, -1);
     s->next_pair = s->last ? NO_PAIR : host_pair(ctx->ph, at, L);
-    const long long tiles = (L + PP_TILE - 1) / PP_TILE;
     int rc;
-    if ((rc = grow(ctx, ctx->tmp[T_PID], (size_t)L * 2 + 64)) ||
-        (rc = grow(ctx, ctx->tmp[T_TSUMS], (tiles + tiles / ST_CHUNK + 2) * sizeof(PosSums))) ||
-        (rc = grow(ctx, ctx->tmp[T_NODEOFF], 16)) || (rc = grow(ctx, ctx->tmp[T_BROFF], 16)))
+    if ((rc = grow(ctx, ctx->tmp[T_PID], (size_t)L * 2 + 64)) || (rc = grow(ctx, ctx->tmp[T_NODEOFF], 16)) || (rc = grow(ctx, ctx->tmp[T_BROFF], 16)))
         return rc;
-    AlpResult* d_res = reinterpret_cast<AlpResult*>(ctx->scratch.p);
-    if ((rc = set_result(ctx, d_res, 1))) return rc;
+    AlpResult* d_res;
+    ScanSync sy;
+    if ((rc = positions_head(ctx, L, &d_res, &sy))) return rc;
     ParseArgs a;
     shard_args(s, a, d_res);
     long long first_pair = NO_PAIR;
     if (L > 0) {
-        const size_t sm1 = pairs_smem_bytes(ctx->pt.n_pairs, ctx->pt.q + ctx->pt.k);
-        const void* fn = pairs_kernel_for(ctx->pt.q, ctx->pt.k);
-        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
-        int sms = 0, per1 = 0;
-        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, fn, PP_THREADS, sm1));
-        const long long x = (long long)persistent_ctas(per1, ctx->tune.pairs_ctas) * sms;
-        {
-            void* args[] = {&a};
-            CK(cudaLaunchKernel(fn, dim3((unsigned)(x < tiles ? x : tiles)), dim3(PP_THREADS), args, sm1, ctx->stream));
-        }
-        const long long chunks = (tiles + ST_CHUNK - 1) / ST_CHUNK;
-        PosSums* csum = a.tile_sums + tiles;
-        scan_tiles_reduce_kernel<<<(unsigned)chunks, ST_CHUNK, 0, ctx->stream>>>(a.tile_sums, tiles, csum, nullptr);
-        CK(cudaGetLastError());
-        scan_tiles_kernel<<<(unsigned)chunks, ST_CHUNK, 0, ctx->stream>>>(a.tile_sums, tiles, csum, d_res, a.node_off,
-                                                                         a.br_off, 1, nullptr);
-        CK(cudaGetLastError());
+        if ((rc = position_sums(ctx, a, sy, 1))) return rc;
         uint16_t p0 = NO_PAIR;
         CK(cudaMemcpyAsync(ctx->h_stage, a.pid, 2, cudaMemcpyDeviceToHost, ctx->stream));
         if ((rc = read_result(ctx, d_res))) return rc;
@@ -3278,15 +3443,15 @@ int alp_parse_tokens(alp_ctx* ctx, const uint32_t* d_term, const int64_t* d_tsta
         return fail(ctx, ALP_ERR_ARG, "null output");
     if (!ctx->has_parser) return fail(ctx, ALP_ERR_MODE, "these tables have no parser");
     CK(cudaSetDevice(ctx->device));
-    int rc = tokens_in(ctx, d_term, d_tstart, d_tend, m);
+    PosHead head;
+    int rc = tokens_in(ctx, d_term, d_tstart, d_tend, m, &head);
     if (rc) return rc;
     ParseOut o{};
-    uint8_t* dvalid = (uint8_t*)ctx->tmp[T_DVALID].p;
     int64_t N = 0;
-    uint8_t* hv = reinterpret_cast<uint8_t*>(ctx->h_stage) + 200;
-    rc = parse_positions(ctx, m + 2, 1, dvalid, &o, 0, 1, &N, 1, hv);
+    uint8_t v = 0;
+    rc = parse_positions(ctx, m + 2, 1, head.base + SC_VALID, &o, 0, 1, &N, 1, &v, &head);
     if (rc) return rc;
-    *valid = hv[0] ? 1 : 0;
+    *valid = v ? 1 : 0;
     *n_node = *valid ? N : 0;
     *d_parent = o.parent;
     *d_tag = o.tag;
@@ -3303,14 +3468,15 @@ int alp_pre_productions(alp_ctx* ctx, const uint32_t* d_term, int64_t m, uint32_
     if (!d_prod || !n_prod || !valid) return fail(ctx, ALP_ERR_ARG, "null output");
     if (!ctx->has_parser) return fail(ctx, ALP_ERR_MODE, "these tables have no parser");
     CK(cudaSetDevice(ctx->device));
-    int rc = tokens_in(ctx, d_term, nullptr, nullptr, m);
+    PosHead head;
+    int rc = tokens_in(ctx, d_term, nullptr, nullptr, m, &head);
     if (rc) return rc;
     ParseOut o{};
-    uint8_t* dvalid = (uint8_t*)ctx->tmp[T_DVALID].p;
     int64_t N = 0;
-    rc = parse_positions(ctx, m + 2, 1, dvalid, &o, 0, 1, &N, 0);
+    uint8_t v = 0;
+    rc = parse_positions(ctx, m + 2, 1, head.base + SC_VALID, &o, 0, 1, &N, 0, &v, &head);
     if (rc) return rc;
-    if ((rc = read_valid0(ctx, dvalid, valid))) return rc;
+    *valid = v ? 1 : 0;
     *n_prod = *valid ? N : 0;
     *d_prod = o.tag;
     return ALP_OK;
@@ -3490,7 +3656,7 @@ static int spec3_lex(alp_ctx* ctx, const uint16_t* wbf, const float* wf32, int n
     if ((rc = grow(ctx, sb[0], K + 16)) || (rc = grow(ctx, sb[1], K + 16)) || (rc = grow(ctx, sb[4], K * 4 + 16)) ||
         (rc = grow(ctx, sb[5], K * 4 + 16)) || (rc = grow(ctx, sb[10], K * 8 + 16)) || (rc = grow(ctx, sb[11], 64)) ||
         (rc = grow(ctx, sb[12], K + 16)) || (rc = grow(ctx, ctx->tmp[T_TOKOFF], 16)) ||
-        (rc = grow(ctx, ctx->tmp[T_DVALID], 16)) || (rc = put_doc_off(ctx, n)))
+        (rc = grow(ctx, ctx->tmp[T_DVALID], 16)))
         return rc;
     uint8_t* dvalid = (uint8_t*)ctx->tmp[T_DVALID].p;
     int64_t cap = n / 2 + 1024;
@@ -3500,8 +3666,7 @@ static int spec3_lex(alp_ctx* ctx, const uint16_t* wbf, const float* wf32, int n
             return rc;
         cap = (int64_t)(ctx->out[1].bytes / 8);
         Lex3Run r;
-        if ((rc = lex3_prepare(ctx, d_in, n, (const long long*)ctx->tmp[T_DOCOFF].p, 1, 0, ctx->out[0].p,
-                               ctx->out[1].p, ctx->out[2].p, cap, dvalid, r)))
+        if ((rc = lex3_prepare(ctx, d_in, n, nullptr, 1, 0, ctx->out[0].p, ctx->out[1].p, ctx->out[2].p, cap, dvalid, r)))
             return rc;
         SpecArgs sa;
         memset(&sa, 0, sizeof sa);
@@ -3826,43 +3991,29 @@ int alp_parse_batch_host(alp_ctx* ctx, const uint8_t* h_in, const int64_t* h_off
 
 namespace {
 
-// positions of the batch from the token pass; the result block reset for the parser
-__global__ void batch_sizes_kernel(AlpResult* res, long long n_docs, long long* sizes) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    sizes[0] = res->count + 2 * n_docs;
-    sizes[1] = (long long)res->error;
-    res->count = 0;
-    res->valid = 1;
-    res->error = 0;
-    for (int i = 0; i < 8; ++i) res->aux[i] = 0;
-}
-
 // counts[0] nodes, [1] brackets, [2] positions, [3] ALP_DEV_ERR_* bits
-__global__ void batch_status_kernel(const AlpResult* res, const long long* sizes, long long cap_nodes,
-                                    long long cap_brs, long long* counts) {
+__global__ void batch_status_kernel(const AlpResult* lex, const AlpResult* res, long long cap_nodes, long long cap_brs,
+                                    long long* counts) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    unsigned int err = res->error | (unsigned int)sizes[1];
+    unsigned int err = res->error | lex->error;
     if (res->aux[0] > cap_nodes || res->aux[1] > cap_brs) err |= ALP_DEV_ERR_CAPACITY;
     counts[0] = res->aux[0];
     counts[1] = res->aux[1];
-    counts[2] = sizes[0];
+    counts[2] = lex->aux[5];
     counts[3] = (long long)err;
 }
 
 // parse_positions with the position count in device memory (dL), L_cap
 // positions at most, and caller capacities for nodes and brackets.
 int parse_positions_dev(alp_ctx* ctx, long long Lcap, const long long* dL, long long nd, uint8_t* dvalid,
-                        const ParseOut& o, long long cap_nodes, long long cap_brs, long long* node_off) {
-    const long long tiles = (Lcap + PP_TILE - 1) / PP_TILE;
+                        const ParseOut& o, long long cap_nodes, long long cap_brs, long long* node_off, AlpResult* d_res,
+                        ScanSync sy) {
     int rc;
-    if ((rc = grow(ctx, ctx->tmp[T_PID], (size_t)Lcap * 2 + 64)) ||
-        (rc = grow(ctx, ctx->tmp[T_TSUMS], (tiles + tiles / ST_CHUNK + 2) * sizeof(PosSums))) ||
-        (rc = grow(ctx, ctx->tmp[T_BROFF], (size_t)(nd + 1) * 8)) || (rc = grow(ctx, ctx->scratch, 256)) ||
+    if ((rc = grow(ctx, ctx->tmp[T_BROFF], (size_t)(nd + 1) * 8)) ||
         (!ctx->tree && ((rc = grow(ctx, ctx->tmp[T_VBUF], (size_t)cap_nodes * 4 + 8)) ||
                         (rc = grow(ctx, ctx->tmp[T_BRBUF], (size_t)cap_brs * 4 + 8)) ||
                         (rc = grow(ctx, ctx->tmp[T_DSBUF], (size_t)cap_brs * 4 + 8)))))
         return rc;
-    AlpResult* d_res = reinterpret_cast<AlpResult*>(ctx->scratch.p);
     ParseArgs a;
     memset(&a, 0, sizeof a);
     a.t = ctx->pt;
@@ -3872,8 +4023,6 @@ int parse_positions_dev(alp_ctx* ctx, long long Lcap, const long long* dL, long 
     a.L = Lcap;
     a.dL = dL;
     a.n_docs = nd;
-    a.pid = (uint16_t*)ctx->tmp[T_PID].p;
-    a.tile_sums = (PosSums*)ctx->tmp[T_TSUMS].p;
     a.res = d_res;
     a.node_off = node_off;
     a.br_off = (long long*)ctx->tmp[T_BROFF].p;
@@ -3888,41 +4037,25 @@ int parse_positions_dev(alp_ctx* ctx, long long Lcap, const long long* dL, long 
     a.dsbuf = (int32_t*)ctx->tmp[T_DSBUF].p;
     a.cap_nodes = cap_nodes;
     a.cap_brs = cap_brs;
-    int sms = 0, per1 = 0, per2 = 0;
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    const size_t sm1 = pairs_smem_bytes(ctx->pt.n_pairs, ctx->pt.q + ctx->pt.k);
-    if (expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack) > 220 * 1024)
-        return fail(ctx, ALP_ERR_TABLE, "parser tables too large for shared memory");
-    size_t sm2 = 0;
-    if ((rc = expand_smem(ctx, (const void*)parse_expand_kernel<0, 0, false>,
-                          expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack), &a.span_cap, &sm2)))
-        return rc;
-    CK(cudaFuncSetAttribute(pairs_kernel_for(ctx->pt.q, ctx->pt.k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, pairs_kernel_for(ctx->pt.q, ctx->pt.k), PP_THREADS, sm1));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, parse_expand_kernel<0, 0, false>, PP_THREADS, sm2));
-    const long long x1 = (long long)persistent_ctas(per1, ctx->tune.pairs_ctas) * sms,
-                    x2 = (long long)persistent_ctas(per2, ctx->tune.expand_ctas) * sms;
-    {
-        void* args[] = {&a};
-        CK(cudaLaunchKernel(pairs_kernel_for(ctx->pt.q, ctx->pt.k), dim3((unsigned)(x1 < tiles ? x1 : tiles)),
-                            dim3(PP_THREADS), args, sm1, ctx->stream));
-    }
-    {
-        const long long chunks = (tiles + ST_CHUNK - 1) / ST_CHUNK;
-        PosSums* csum = a.tile_sums + tiles;
-        scan_tiles_reduce_kernel<<<(unsigned)chunks, ST_CHUNK, 0, ctx->stream>>>(a.tile_sums, tiles, csum, dL);
-        CK(cudaGetLastError());
-        scan_tiles_kernel<<<(unsigned)chunks, ST_CHUNK, 0, ctx->stream>>>(a.tile_sums, tiles, csum, d_res, a.node_off,
-                                                                         a.br_off, nd, dL);
-        CK(cudaGetLastError());
-    }
+    if ((rc = position_sums(ctx, a, sy, nd))) return rc;
     if (ctx->tree) {
         TreeArgs t = tree_args(ctx, a, (long long*)o.parent);
         if ((rc = run_tree(ctx, t, false))) return rc;
         return run_tree_escapes(ctx, t);
     }
-    parse_expand_kernel<0, 0, false><<<(unsigned)(x2 < tiles ? x2 : tiles), PP_THREADS, sm2, ctx->stream>>>(a);
-    CK(cudaGetLastError());
+    const long long tiles = (Lcap + PP_TILE - 1) / PP_TILE;
+    const void* ex = (const void*)parse_expand_kernel<0, 0, false>;
+    if (expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack) > 220 * 1024)
+        return fail(ctx, ALP_ERR_TABLE, "parser tables too large for shared memory");
+    size_t sm2 = 0;
+    unsigned g2 = 1;
+    if ((rc = expand_smem(ctx, ex, expand_smem_bytes(ctx->pt.n_pairs, ctx->pt.n_pseq, ctx->pt.n_stack), &a.span_cap, &sm2)) ||
+        (rc = expand_grid(ctx, ex, sm2, tiles, &g2)))
+        return rc;
+    {
+        void* args[] = {&a};
+        CK(cudaLaunchKernel(ex, dim3(g2), dim3(PP_THREADS), args, sm2, ctx->stream));
+    }
     if ((rc = run_ple(ctx, a.vbuf, cap_nodes, nullptr, o.parent, T_N_TMIN, a.node_off, nd, dvalid, d_res,
                       &d_res->aux[0])))
         return rc;
@@ -3937,7 +4070,6 @@ struct alp_parse_graph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t last = nullptr;     // stream of the last launch
-    long long* sizes = nullptr;      // device: positions, lexer error bits
     long long* h_counts = nullptr;   // pinned
     int64_t* d_counts = nullptr;
     long long cap_nodes = 0, cap_brs = 0;
@@ -3966,14 +4098,12 @@ int graph_enqueue(alp_parse_graph* g) {
                            ctx->tmp[T_TSTART].p, ctx->tmp[T_TEND].p, (long long)tcap, g->d_valid, r)) ||
         (rc = lex3_front(ctx, r)) || (rc = lex3_emit<uint16_t, uint32_t>(ctx, r)))
         return rc;
-    AlpResult* d_res = reinterpret_cast<AlpResult*>(ctx->scratch.p);
-    batch_sizes_kernel<<<1, 32, 0, ctx->stream>>>(d_res, nd, g->sizes);
-    CK(cudaGetLastError());
-    if ((rc = parse_positions_dev(ctx, n + 2 * nd, g->sizes, nd, g->d_valid, g->o, g->cap_nodes, g->cap_brs,
-                                  (long long*)g->d_node_off)))
+    // (positions of the batch: the tile scan's total in the lexer's result)
+    AlpResult* d_res = reinterpret_cast<AlpResult*>(r.base + SC_PARSE);
+    if ((rc = parse_positions_dev(ctx, n + 2 * nd, &r.a.res->aux[5], nd, g->d_valid, g->o, g->cap_nodes, g->cap_brs,
+                                  (long long*)g->d_node_off, d_res, r.pos_sync)))
         return rc;
-    batch_status_kernel<<<1, 32, 0, ctx->stream>>>(d_res, g->sizes, g->cap_nodes, g->cap_brs,
-                                                   (long long*)g->d_counts);
+    batch_status_kernel<<<1, 32, 0, ctx->stream>>>(r.a.res, d_res, g->cap_nodes, g->cap_brs, (long long*)g->d_counts);
     CK(cudaGetLastError());
     return ALP_OK;
 }
@@ -4005,7 +4135,6 @@ void graph_free(alp_parse_graph* g) {
     if (g->child) cudaSetDevice(g->child->device);
     if (g->exec) cudaGraphExecDestroy(g->exec);
     if (g->graph) cudaGraphDestroy(g->graph);
-    if (g->sizes) cudaFree(g->sizes);
     if (g->h_counts) cudaFreeHost(g->h_counts);
     if (g->child) {
         g->child->stream = nullptr;
@@ -4046,8 +4175,8 @@ int alp_parse_graph_create(alp_ctx* ctx, const uint8_t* d_in, int64_t n, const i
         return fail(ctx, rc, "%s", m.c_str());
     };
     if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&g->sizes, 64) != cudaSuccess || cudaMallocHost(&g->h_counts, 64) != cudaSuccess ||
-        cudaMallocHost(&g->child->h_res, sizeof(AlpResult)) != cudaSuccess ||
+        cudaMallocHost(&g->h_counts, 64) != cudaSuccess ||
+        cudaMallocHost(&g->child->h_res, SC_COPY) != cudaSuccess ||
         cudaMallocHost(&g->child->h_stage, 256) != cudaSuccess)
         return bad(ALP_ERR_CUDA, "graph set-up failed");
     g->child->stream = g->stream;

@@ -19,8 +19,7 @@
 //                      carry the produce/ignore decisions, and stores the chunk's
 //                      token count, last token start and a record per token
 //                      (lexwalk.cuh).
-//   lex3_tile_reduce_kernel, lex3_tile_scan_kernel  exclusive (count, last
-//                      start) over 8 KiB tiles, the
+//   lex3_tile_scan_kernel  exclusive (count, last start) over 8 KiB tiles, the
 //                      take_right start scan and the compaction offsets
 //                      (futhark/lexer.fut:83-84,108-120) at tile level.
 //   lex3_write_kernel  the compaction (futhark/lexer.fut:121-133): places each
@@ -512,55 +511,34 @@ __device__ __forceinline__ void cs_reduce_warp(uint32_t& c, uint32_t& p) {
 }
 
 // ---- kernel 4: exclusive (count, last start) over tiles ---------------------
-// Two launches over chunks of LT_CHUNK tiles: the chunk sums, then one CTA per
-// chunk scans the chunk sums before its own and its own tiles in place.
-// Tile 0 starts from (0, NONE): no token start before the input.
+// One launch over chunks of LT_CHUNK tiles, one CTA each: a chunk publishes its sum and
+// waits for those of the chunks before it (in ticket order, so all of them are running or
+// done), then scans its own tiles in place.  A second launch for the chunk sums cost 3 to
+// 6 us of every call.  Tile 0 starts from (0, NONE): no token start before the input.
+// The totals: res->aux[6] tokens, aux[5] parser positions (two more per document).
 constexpr int LT_CHUNK = 1024;
+
+struct ScanSync {
+    unsigned int* ticket;   // zero before the launch
+    uint32_t* flag;         // [chunks] zero before the launch
+    void* sums;             // [chunks] of the scanned type
+};
 
 __device__ __forceinline__ void cs_unpack(unsigned long long v, uint32_t& c, uint32_t& p) {
     c = (uint32_t)(v >> 32);
     p = (uint32_t)v;
 }
 
-__global__ void __launch_bounds__(LT_CHUNK) lex3_tile_reduce_kernel(const unsigned long long* tile_cs, long long T,
-                                                                    unsigned long long* chunk_cs) {
+__global__ void __launch_bounds__(LT_CHUNK) lex3_tile_scan_kernel(unsigned long long* tile_cs, long long T, ScanSync sy,
+                                                                  long long extra, AlpResult* res) {
     __shared__ uint32_t s_c[LT_CHUNK / 32], s_p[LT_CHUNK / 32];
+    __shared__ uint32_t s_cc, s_cp, s_chunk;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const long long i = (long long)blockIdx.x * LT_CHUNK + tid;
-    uint32_t c = 0, p = ALP_NONE32;
-    if (i < T) cs_unpack(tile_cs[i], c, p);
-    cs_reduce_warp(c, p);
-    if (lane == 0) { s_c[warp] = c; s_p[warp] = p; }
+    if (tid == 0) s_chunk = gridDim.x > 1 ? atomicAdd(sy.ticket, 1u) : 0u;
     __syncthreads();
-    if (tid == 0) {
-        uint32_t tc = 0, tp = ALP_NONE32;
-        for (int w = 0; w < LT_CHUNK / 32; ++w) {
-            tc += s_c[w];
-            if (s_p[w] != ALP_NONE32) tp = s_p[w];
-        }
-        chunk_cs[blockIdx.x] = ((unsigned long long)tc << 32) | tp;
-    }
-}
-
-__global__ void __launch_bounds__(LT_CHUNK) lex3_tile_scan_kernel(unsigned long long* tile_cs, long long T,
-                                                                  const unsigned long long* chunk_cs, AlpResult* res) {
-    __shared__ uint32_t s_c[LT_CHUNK / 32], s_p[LT_CHUNK / 32];
-    __shared__ uint32_t s_cc, s_cp;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const long long chunk = blockIdx.x;
-    if (warp == 0) {
-        uint32_t cc = 0, cp = ALP_NONE32;
-        for (long long b = 0; b < chunk; b += 32) {
-            uint32_t c = 0, p = ALP_NONE32;
-            if (b + lane < chunk) cs_unpack(chunk_cs[b + lane], c, p);
-            cs_reduce_warp(c, p);
-            c = __shfl_sync(ALP_FULL_MASK, c, 0);
-            p = __shfl_sync(ALP_FULL_MASK, p, 0);
-            cc += c;
-            if (p != ALP_NONE32) cp = p;
-        }
-        if (lane == 0) { s_cc = cc; s_cp = cp; }
-    }
+    const long long chunk = s_chunk;
+    if (chunk * LT_CHUNK >= T) return;
+    unsigned long long* sums = reinterpret_cast<unsigned long long*>(sy.sums);
     const long long i = chunk * LT_CHUNK + tid;
     uint32_t c = 0, p = ALP_NONE32;
     if (i < T) cs_unpack(tile_cs[i], c, p);
@@ -571,6 +549,29 @@ __global__ void __launch_bounds__(LT_CHUNK) lex3_tile_scan_kernel(unsigned long 
     if (warp == 0) {
         uint32_t wc = s_c[lane], wp = s_p[lane];
         warp_scan_cs(wc, wp, lane);
+        uint32_t cc = 0, cp = ALP_NONE32;
+        if (gridDim.x > 1) {
+            if (lane == 31) {
+                *reinterpret_cast<volatile unsigned long long*>(sums + chunk) = ((unsigned long long)wc << 32) | wp;
+                __threadfence();
+                st_volatile32(&sy.flag[chunk], ST_A << 30);
+            }
+            for (long long b = 0; b < chunk; b += 32) {
+                uint32_t xc = 0, xp = ALP_NONE32;
+                if (b + lane < chunk) {
+                    wait32(&sy.flag[b + lane], &res->error);
+                    __threadfence();
+                    cs_unpack(ld_volatile64(sums + b + lane), xc, xp);
+                }
+                __syncwarp();
+                cs_reduce_warp(xc, xp);
+                xc = __shfl_sync(ALP_FULL_MASK, xc, 0);
+                xp = __shfl_sync(ALP_FULL_MASK, xp, 0);
+                cc += xc;
+                if (xp != ALP_NONE32) cp = xp;
+            }
+        }
+        if (lane == 0) { s_cc = cc; s_cp = cp; }
         uint32_t xc = __shfl_up_sync(ALP_FULL_MASK, wc, 1), xp = __shfl_up_sync(ALP_FULL_MASK, wp, 1);
         if (lane == 0) { xc = 0; xp = ALP_NONE32; }
         s_c[lane] = xc;
@@ -582,7 +583,11 @@ __global__ void __launch_bounds__(LT_CHUNK) lex3_tile_scan_kernel(unsigned long 
     const uint32_t rc = s_cc + s_c[warp] + ec;
     uint32_t rp = ep != ALP_NONE32 ? ep : (s_p[warp] != ALP_NONE32 ? s_p[warp] : s_cp);
     if (i < T) tile_cs[i] = ((unsigned long long)rc << 32) | rp;
-    if (i == T - 1) res->aux[6] = (long long)rc + c;  // all tokens
+    if (i == T - 1) {
+        res->aux[6] = (long long)rc + c;
+        // a front that timed out has no positions for the parser kernels behind it
+        res->aux[5] = *reinterpret_cast<volatile unsigned int*>(&res->error) ? 0 : (long long)rc + c + extra;
+    }
 }
 
 // ---- kernel 5: tokens ---------------------------------------------------------

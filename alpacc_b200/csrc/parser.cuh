@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "lex3.cuh"
 
 namespace alp {
 
@@ -392,6 +393,7 @@ __global__ void __launch_bounds__(PP_THREADS, 3) parse_pairs_kernel(ParseArgs a)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int q = QT > 0 ? QT : a.t.q, k = KT > 0 ? KT : a.t.k, W = q + k;
     if (a.dL) a.L = *a.dL;
+    if ((long long)blockIdx.x * PP_TILE >= a.L) return;  // with dL the grid covers the capacity
     for (int i = tid; i < a.t.n_pairs * (int)(sizeof(PairInfo) / 4); i += PP_THREADS)
         reinterpret_cast<uint32_t*>(s_pi)[i] = reinterpret_cast<const uint32_t*>(a.t.pairs)[i];
     if (tid == 0) {
@@ -552,116 +554,122 @@ inline const void* pairs_kernel_for(int q, int k) {
     return (const void*)parse_pairs_kernel<0, 0>;
 }
 
-// Exclusive segmented scan of the tile sums in place, in two launches:
-// scan_tiles_reduce_kernel sums each chunk of ST_CHUNK tiles, then
-// scan_tiles_kernel (one CTA per chunk) scans the chunk sums before its own
-// and its own tiles.  Totals go to res->aux (nodes, brackets, final depth, -,
-// -, heads) and the closing entries of node_off / br_off.
+// Exclusive segmented scan of the tile sums in place, in one launch over chunks of ST_CHUNK
+// tiles, as lex3_tile_scan_kernel: a chunk publishes its sum, waits for those before it and
+// scans its own tiles.  Totals go to res->aux (nodes, brackets, final depth, -, -, heads)
+// and the closing entries of node_off / br_off.  (A launch of its own for the chunk sums cost
+// 6 us of every call.)
 constexpr int ST_CHUNK = 1024;
 
-__device__ __forceinline__ PosSums ps_block_reduce(PosSums v, PosSums* s_w) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    PosSums inc = ps_warp_scan(v, lane);
-    if (lane == 31) s_w[warp] = inc;
-    __syncthreads();
-    PosSums t = s_w[0];
-    for (int w = 1; w < (int)(blockDim.x / 32); ++w) t = ps_combine(t, s_w[w]);
-    return t;
+__device__ __forceinline__ PosSums ps_shfl(const PosSums& x, int src) {
+    PosSums r;
+    r.nodes = __shfl_sync(ALP_FULL_MASK, x.nodes, src);
+    r.brs = __shfl_sync(ALP_FULL_MASK, x.brs, src);
+    r.depth = __shfl_sync(ALP_FULL_MASK, x.depth, src);
+    r.v = __shfl_sync(ALP_FULL_MASK, x.v, src);
+    r.terms = __shfl_sync(ALP_FULL_MASK, x.terms, src);
+    r.heads = __shfl_sync(ALP_FULL_MASK, x.heads, src);
+    r.hpos = __shfl_sync(ALP_FULL_MASK, x.hpos, src);
+    r.cls = __shfl_sync(ALP_FULL_MASK, x.cls, src);
+    r.dnodes = __shfl_sync(ALP_FULL_MASK, x.dnodes, src);
+    return r;
+}
+// sums as another CTA wrote them, past this SM's L1
+__device__ __forceinline__ PosSums ps_ld(const PosSums* p) {
+    const volatile uint4* v = reinterpret_cast<const volatile uint4*>(p);
+    const uint4 x = make_uint4(v[0].x, v[0].y, v[0].z, v[0].w), y = make_uint4(v[1].x, v[1].y, v[1].z, v[1].w);
+    PosSums r;
+    r.nodes = x.x; r.brs = x.y; r.depth = (int32_t)x.z; r.v = (int32_t)x.w;
+    r.terms = y.x; r.heads = y.y; r.hpos = (int32_t)y.z; r.cls = y.w;
+    r.dnodes = v[2].x;
+    return r;
+}
+__device__ __forceinline__ void ps_st(PosSums* p, const PosSums& r) {
+    volatile uint4* v = reinterpret_cast<volatile uint4*>(p);
+    v[0].x = r.nodes; v[0].y = r.brs; v[0].z = (uint32_t)r.depth; v[0].w = (uint32_t)r.v;
+    v[1].x = r.terms; v[1].y = r.heads; v[1].z = (uint32_t)r.hpos; v[1].w = r.cls;
+    v[2].x = r.dnodes;
 }
 
-__global__ void __launch_bounds__(ST_CHUNK) scan_tiles_reduce_kernel(const PosSums* s, long long tiles,
-                                                                     PosSums* chunk_sums, const long long* dL) {
-    __shared__ PosSums s_w[ST_CHUNK / 32];
-    if (dL) tiles = (*dL + PP_TILE - 1) / PP_TILE;  // the grid covers the capacity
-    const long long idx = (long long)blockIdx.x * ST_CHUNK + threadIdx.x;
-    PosSums v;
-    if (idx < tiles) v = s[idx]; else possums_zero(v);
-    const PosSums t = ps_block_reduce(v, s_w);
-    if (threadIdx.x == 0) chunk_sums[blockIdx.x] = t;
-}
-
-__global__ void __launch_bounds__(ST_CHUNK) scan_tiles_kernel(PosSums* s, long long tiles, const PosSums* chunk_sums,
-                                                              AlpResult* res, long long* node_off, long long* br_off,
-                                                              long long n_docs, const long long* dL) {
+__global__ void __launch_bounds__(ST_CHUNK) scan_tiles_kernel(PosSums* s, long long tiles, ScanSync sy, AlpResult* res,
+                                                              long long* node_off, long long* br_off, long long n_docs,
+                                                              const long long* dL) {
     __shared__ PosSums s_w[ST_CHUNK / 32];
     __shared__ PosSums s_carry;
+    __shared__ uint32_t s_chunk;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const long long chunk = blockIdx.x;
     if (dL) tiles = (*dL + PP_TILE - 1) / PP_TILE;  // the grid covers the capacity
     const long long last = (tiles + ST_CHUNK - 1) / ST_CHUNK - 1;
+    if (tid == 0) s_chunk = gridDim.x > 1 ? atomicAdd(sy.ticket, 1u) : 0u;
+    __syncthreads();
+    const long long chunk = s_chunk;
     if (chunk > last) return;
-    if (warp == 0) {
-        PosSums carry;
-        possums_zero(carry);
-        for (long long b = 0; b < chunk; b += 32) {
-            PosSums v;
-            if (b + lane < chunk) v = chunk_sums[b + lane]; else possums_zero(v);
-            const PosSums inc = ps_warp_scan(v, lane);
-            PosSums last;
-            last.nodes = __shfl_sync(ALP_FULL_MASK, inc.nodes, 31);
-            last.brs = __shfl_sync(ALP_FULL_MASK, inc.brs, 31);
-            last.depth = __shfl_sync(ALP_FULL_MASK, inc.depth, 31);
-            last.v = __shfl_sync(ALP_FULL_MASK, inc.v, 31);
-            last.terms = __shfl_sync(ALP_FULL_MASK, inc.terms, 31);
-            last.heads = __shfl_sync(ALP_FULL_MASK, inc.heads, 31);
-            last.hpos = __shfl_sync(ALP_FULL_MASK, inc.hpos, 31);
-            last.cls = __shfl_sync(ALP_FULL_MASK, inc.cls, 31);
-            last.dnodes = __shfl_sync(ALP_FULL_MASK, inc.dnodes, 31);
-            carry = ps_combine(carry, last);
-        }
-        if (lane == 0) s_carry = carry;
-    }
+    PosSums* sums = reinterpret_cast<PosSums*>(sy.sums);
     const long long idx = chunk * ST_CHUNK + tid;
     PosSums v;
     if (idx < tiles) v = s[idx]; else possums_zero(v);
-    PosSums inc = ps_warp_scan(v, lane);
+    const PosSums inc = ps_warp_scan(v, lane);
     PosSums ex = ps_shfl_up(inc, 1);
     if (lane == 0) possums_zero(ex);
     if (lane == 31) s_w[warp] = inc;
     __syncthreads();
     if (warp == 0) {
-        PosSums w = s_w[lane];
-        PosSums wi = ps_warp_scan(w, lane);
+        const PosSums wi = ps_warp_scan(s_w[lane], lane);
         PosSums we = ps_shfl_up(wi, 1);
         if (lane == 0) possums_zero(we);
+        __syncwarp();
         s_w[lane] = we;
-    }
-    __syncthreads();
-    const PosSums pre = ps_combine(s_carry, s_w[warp]);
-    if (idx < tiles) s[idx] = ps_combine(pre, ex);
-    if (chunk == last) {
-        __syncthreads();
-        if (tid == ST_CHUNK - 1) s_carry = ps_combine(pre, inc);
-        if (warp == 0) {
-            // node, bracket and closed-pair totals in 64 bits, so that a total past 2^32 is seen
-            unsigned long long tn = 0, tb = 0, tc = 0;
-            for (long long b = lane; b <= chunk; b += 32) {
-                if (b < chunk) { tn += chunk_sums[b].nodes; tb += chunk_sums[b].brs; tc += chunk_sums[b].cls; }
+        PosSums carry;
+        possums_zero(carry);
+        // node, bracket and closed-pair totals in 64 bits, so that a total past 2^32 is seen
+        unsigned long long tn = 0, tb = 0, tc = 0;
+        if (last > 0) {
+            if (lane == 31) {
+                ps_st(sums + chunk, wi);
+                __threadfence();
+                st_volatile32(&sy.flag[chunk], ST_A << 30);
             }
+            for (long long b = 0; b < chunk; b += 32) {
+                PosSums x;
+                possums_zero(x);
+                if (b + lane < chunk) {
+                    wait32(&sy.flag[b + lane], &res->error);
+                    __threadfence();
+                    x = ps_ld(sums + b + lane);
+                }
+                __syncwarp();
+                tn += x.nodes;
+                tb += x.brs;
+                tc += x.cls;
+                carry = ps_combine(carry, ps_shfl(ps_warp_scan(x, lane), 31));
+            }
+        }
+        if (lane == 0) s_carry = carry;
+        if (chunk == last) {
+            if (lane == 31) { tn += wi.nodes; tb += wi.brs; tc += wi.cls; }
             for (int d = 16; d >= 1; d >>= 1) {
                 tn += __shfl_down_sync(ALP_FULL_MASK, tn, d);
                 tb += __shfl_down_sync(ALP_FULL_MASK, tb, d);
                 tc += __shfl_down_sync(ALP_FULL_MASK, tc, d);
             }
-            if (lane == 0) { res->aux[0] = (long long)tn; res->aux[1] = (long long)tb; res->aux[7] = (long long)tc; }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            const PosSums tot = s_carry;
-            // the last chunk's own sums on top of the 64-bit totals of the earlier chunks
-            const PosSums own = chunk_sums[chunk];
-            res->aux[0] += own.nodes;
-            res->aux[1] += own.brs;
-            res->aux[7] += own.cls;
-            res->aux[2] = tot.depth;
-            res->aux[3] = tot.v;
-            res->aux[4] = (long long)tot.terms;
-            res->aux[5] = (long long)tot.heads;
-            res->aux[6] = res->aux[1] - 2 * res->aux[7];  // brackets left for the search
-            node_off[n_docs] = res->aux[0];
-            br_off[n_docs] = res->aux[6];
+            const PosSums tot = ps_combine(carry, ps_shfl(wi, 31));
+            if (lane == 0) {
+                res->aux[0] = (long long)tn;
+                res->aux[1] = (long long)tb;
+                res->aux[2] = tot.depth;
+                res->aux[3] = tot.v;
+                res->aux[4] = (long long)tot.terms;
+                res->aux[5] = (long long)tot.heads;
+                res->aux[6] = (long long)(tb - 2 * tc);  // brackets left for the search
+                res->aux[7] = (long long)tc;
+                node_off[n_docs] = (long long)tn;
+                br_off[n_docs] = (long long)(tb - 2 * tc);
+            }
         }
     }
+    __syncthreads();
+    const PosSums pre = ps_combine(s_carry, s_w[warp]);
+    if (idx < tiles) s[idx] = ps_combine(pre, ex);
 }
 
 // ---------------------------------------------------------------------------
@@ -743,21 +751,6 @@ __device__ __forceinline__ void ex_words(const ParseArgs& a, long long i0, uint2
 // it meets an inclusive prefix, and publishes this tile's inclusive prefix.
 // Payloads are written before their flag with a fence in between; a reader
 // fences after it sees the flag.
-__device__ __forceinline__ PosSums ps_ld(const PosSums* p) {
-    const volatile uint4* v = reinterpret_cast<const volatile uint4*>(p);
-    const uint4 x = make_uint4(v[0].x, v[0].y, v[0].z, v[0].w), y = make_uint4(v[1].x, v[1].y, v[1].z, v[1].w);
-    PosSums r;
-    r.nodes = x.x; r.brs = x.y; r.depth = (int32_t)x.z; r.v = (int32_t)x.w;
-    r.terms = y.x; r.heads = y.y; r.hpos = (int32_t)y.z; r.cls = y.w;
-    r.dnodes = v[2].x;
-    return r;
-}
-__device__ __forceinline__ void ps_st(PosSums* p, const PosSums& r) {
-    volatile uint4* v = reinterpret_cast<volatile uint4*>(p);
-    v[0].x = r.nodes; v[0].y = r.brs; v[0].z = (uint32_t)r.depth; v[0].w = (uint32_t)r.v;
-    v[1].x = r.terms; v[1].y = r.heads; v[1].z = (uint32_t)r.hpos; v[1].w = r.cls;
-    v[2].x = r.dnodes;
-}
 __device__ __forceinline__ PosSums ps_shfl_down(const PosSums& x, int d) {
     PosSums r;
     r.nodes = __shfl_down_sync(ALP_FULL_MASK, x.nodes, d);

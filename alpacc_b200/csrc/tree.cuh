@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_tree_kernel(TreeArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = PP_THREADS / 32;
     if (a.dL) a.L = *a.dL;
+    if ((long long)blockIdx.x * PP_TILE >= a.L) return;  // with dL the grid covers the capacity
     for (int i = tid; i <= a.t.n_pairs; i += PP_THREADS) s_pr[i] = a.t.pairs[i];
     for (int i = tid; i < a.t.n_pseq; i += PP_THREADS) s_rec[i] = a.t.rec[i];
     for (int i = tid; i < a.t.n_stack; i += PP_THREADS) s_se[i] = a.t.stack[i];
