@@ -39,6 +39,8 @@ constexpr int LX_TILE = LX_THREADS * LX_CHUNK;  // 8 KiB emit tile: one chunk pe
 constexpr int LX_WIDE = 2 * LX_TILE;            // 16 KiB fold / walk tile: two chunks per thread
 constexpr int LX_STAGE = 2048;                  // tokens one emit tile stages in shared memory
 constexpr int LS_WARPS = 8;
+constexpr int LS_BACK = 4;                      // tiles a look-back step of the state scan loads at once
+constexpr int LS_CHAINS = 4;                    // runs of units a warp follows side by side
 constexpr int LS_G = 16;                        // chunks per lane in the state scan (default; 8, 16 or 32)
 __host__ __device__ constexpr long long ls_tile(int g) { return (long long)LS_WARPS * 32 * g; }  // chunks per scan tile
 
@@ -331,14 +333,21 @@ __global__ void __launch_bounds__(LX_THREADS, 4) lex3_fold_kernel(Lex3Args a, Le
 }
 
 // ---- kernel 2: states entering the chunks -----------------------------------
-// G chunks per lane (a tuned launch shape: 8, 16 or 32).
+// G units per lane (a tuned launch shape: 8, 16 or 32).  A warp's 32 * G units are followed
+// from every state, a lane a state: dependent table lookups of some 30 cycles each, which one
+// tile waits for and many tiles hide.  So the units are LS_CHAINS runs followed side by side,
+// joined by one lookup per lane; their numbers come from shared memory, eight to a broadcast
+// load, where a shuffle for each two took a third of the shared-memory pipe.
+// One tile (a small call) 12.5 -> 8.5 us; 256 MiB stays at 51.
 template <int G>
 __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
     static_assert(G == 8 || G == 16 || G == 32, "chunks per lane");
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t rows = (uint32_t)(a.t.E + a.t.S);
     uint8_t* s_app = smem;
-    __shared__ uint8_t s_sv[LS_WARPS][32][32];  // [warp][lane segment][start state] -> state
+    __shared__ uint4 s_f[LS_WARPS][32][G / 8];  // unit numbers: [warp][lane segment], 16 bits each
+    __shared__ uint8_t s_sv[LS_WARPS][32][32];  // [warp][lane segment][state at its run's start] -> state
+    __shared__ uint8_t s_run[LS_WARPS][LS_CHAINS][32];  // [warp][run][state before the warp's units] -> state
     __shared__ uint8_t s_wagg[LS_WARPS][32];
     __shared__ uint8_t s_wpre[LS_WARPS][32];
     __shared__ uint32_t s_tile, s_sin;
@@ -358,36 +367,56 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
         if (tile >= a.num_scan_tiles) break;
         const long long base = (long long)tile * ls_tile(G) + (long long)warp * (32 * G) + (long long)lane * G;
 
-        // this lane's G chunk endomorphisms, two per word
-        uint32_t fr[G / 2];
+        // this lane's G unit endomorphisms
         if (base + G <= M) {
             const uint4* p = reinterpret_cast<const uint4*>(a.unit_f + base);
 #pragma unroll
-            for (int v = 0; v < G / 8; ++v) {
-                const uint4 x = p[v];
-                fr[4 * v] = x.x; fr[4 * v + 1] = x.y; fr[4 * v + 2] = x.z; fr[4 * v + 3] = x.w;
-            }
+            for (int v = 0; v < G / 8; ++v) s_f[warp][lane][v] = p[v];
         } else {
 #pragma unroll
-            for (int q = 0; q < G / 2; ++q) {
-                const uint32_t lo = base + 2 * q < M ? a.unit_f[base + 2 * q] : 0u;
-                const uint32_t hi = base + 2 * q + 1 < M ? a.unit_f[base + 2 * q + 1] : 0u;
-                fr[q] = lo | (hi << 16);
-            }
-        }
-
-        // lane s follows state s through the warp's 512 chunks
-        uint32_t cur = (uint32_t)lane;
-        for (int l2 = 0; l2 < 32; ++l2) {
-            s_sv[warp][l2][lane] = (uint8_t)cur;
+            for (int v = 0; v < G / 8; ++v) {
+                uint32_t x[4];
 #pragma unroll
-            for (int q = 0; q < G / 2; ++q) {
-                const uint32_t v = __shfl_sync(ALP_FULL_MASK, fr[q], l2);
-                cur = s_app[(v & 0xffffu) * 32 + cur];
-                cur = s_app[(v >> 16) * 32 + cur];
+                for (int q = 0; q < 4; ++q) {
+                    const long long at = base + 8 * v + 2 * q;
+                    x[q] = (at < M ? a.unit_f[at] : 0u) | ((at + 1 < M ? a.unit_f[at + 1] : 0u) << 16);
+                }
+                s_f[warp][lane][v] = make_uint4(x[0], x[1], x[2], x[3]);
             }
         }
-        s_wagg[warp][lane] = (uint8_t)cur;
+        __syncwarp();
+
+        // lane s follows state s through each run of the warp's units
+        constexpr int RUN = 32 / LS_CHAINS;  // lane segments of a run
+        uint32_t cur[LS_CHAINS];
+#pragma unroll
+        for (int c = 0; c < LS_CHAINS; ++c) cur[c] = (uint32_t)lane;
+#pragma unroll 1
+        for (int l2 = 0; l2 < RUN; ++l2) {
+#pragma unroll
+            for (int c = 0; c < LS_CHAINS; ++c) s_sv[warp][c * RUN + l2][lane] = (uint8_t)cur[c];
+#pragma unroll
+            for (int v = 0; v < G / 8; ++v) {
+                uint4 f[LS_CHAINS];
+#pragma unroll
+                for (int c = 0; c < LS_CHAINS; ++c) f[c] = s_f[warp][c * RUN + l2][v];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+#pragma unroll
+                    for (int c = 0; c < LS_CHAINS; ++c) {
+                        const uint32_t w = q < 2 ? f[c].x : (q < 4 ? f[c].y : (q < 6 ? f[c].z : f[c].w));
+                        cur[c] = s_app[((q & 1) ? (w >> 16) : (w & 0xffffu)) * 32 + cur[c]];
+                    }
+                }
+            }
+        }
+        uint32_t through = (uint32_t)lane;  // lane s: the state from s after the runs so far
+#pragma unroll
+        for (int c = 0; c < LS_CHAINS; ++c) {
+            s_run[warp][c][lane] = (uint8_t)through;
+            through = __shfl_sync(ALP_FULL_MASK, cur[c], through & 31u);
+        }
+        s_wagg[warp][lane] = (uint8_t)through;
         __syncthreads();
 
         if (warp == 0) {
@@ -405,13 +434,13 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
                 long long j = (long long)tile - 1;
                 bool done = false;
                 while (!done) {
-                    uint32_t wv[4];
+                    uint32_t wv[LS_BACK];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
+                    for (int q = 0; q < LS_BACK; ++q)
                         wv[q] = j - q >= 0 ? ld_volatile32(&a.lb_vec[(size_t)(j - q) * 32 + lane])
                                            : ((ST_P << 30) | INIT);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
+                    for (int q = 0; q < LS_BACK; ++q) {
                         if (!done) {
                             uint32_t wq = wv[q];
                             if ((wq >> 30) == ST_X) wq = wait32(&a.lb_vec[(size_t)(j - q) * 32 + lane], &a.res->error);
@@ -426,7 +455,7 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
                             }
                         }
                     }
-                    j -= 4;
+                    j -= LS_BACK;
                 }
             }
             const uint32_t out = __shfl_sync(ALP_FULL_MASK, x, sin & 31u);
@@ -436,16 +465,19 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
         __syncthreads();
 
         const uint32_t win = s_wpre[warp][s_sin & 31u];
-        uint32_t st = s_sv[warp][lane][win];
+        uint32_t st = s_sv[warp][lane][s_run[warp][lane / RUN][win]];
         uint32_t ob[G / 4];
 #pragma unroll
         for (int q = 0; q < G / 4; ++q) ob[q] = 0;
 #pragma unroll
-        for (int q = 0; q < G / 2; ++q) {
-            ob[q >> 1] |= st << (16 * (q & 1));
-            st = s_app[(fr[q] & 0xffffu) * 32 + st];
-            ob[q >> 1] |= st << (16 * (q & 1) + 8);
-            st = s_app[(fr[q] >> 16) * 32 + st];
+        for (int v = 0; v < G / 8; ++v) {
+            const uint4 f = s_f[warp][lane][v];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const uint32_t w = q < 2 ? f.x : (q < 4 ? f.y : (q < 6 ? f.z : f.w));
+                ob[2 * v + (q >> 2)] |= st << (8 * (q & 3));
+                st = s_app[((q & 1) ? (w >> 16) : (w & 0xffffu)) * 32 + st];
+            }
         }
         if (base + G <= M) {
             if constexpr (G == 8) {
