@@ -274,6 +274,7 @@ __global__ void __launch_bounds__(LX_THREADS, 4) lex3_fold_kernel(Lex3Args a, Le
         const int words = (int)((2 * (size_t)(E + S) * C1 + 15) / 16);
         for (int i = tid; i < words; i += LX_THREADS) reinterpret_cast<uint4*>(s_step)[i] = __ldg(src + i);
     }
+    after_prior_kernel();
     const uint32_t unit = F2 ? 2u * (uint32_t)C1 : 1u;
     const uint32_t init = (E + 1u) * unit;
     // endomorphism number of a fold value: exact for values below 2^16 (umulhi by ceil(2^32 / unit))
@@ -358,6 +359,7 @@ __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
         uint4* dst = reinterpret_cast<uint4*>(s_app);
         for (uint32_t i = tid; i < rows * 2; i += LS_WARPS * 32) dst[i] = src[i];
     }
+    after_prior_kernel();
     const uint32_t INIT = 1u;
     const long long M = a.n_units;
     for (;;) {
@@ -566,6 +568,7 @@ __global__ void __launch_bounds__(LT_CHUNK) lex3_tile_scan_kernel(unsigned long 
     __shared__ uint32_t s_c[LT_CHUNK / 32], s_p[LT_CHUNK / 32];
     __shared__ uint32_t s_cc, s_cp, s_chunk;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    after_prior_kernel();
     if (tid == 0) s_chunk = gridDim.x > 1 ? atomicAdd(sy.ticket, 1u) : 0u;
     __syncthreads();
     const long long chunk = s_chunk;

@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(LX_THREADS, 6) lex3_walk_kernel(Lex3Args a, Le
         for (int i = tid; i < words; i += LX_THREADS) dst[i] = __ldg(src + i);
     }
     if (tid < S) s_tok[tid] = a.t.tokinfo[tid];
+    after_prior_kernel();
     const uint32_t ro = (uint32_t)lw_table_bytes(S) + tid * 2 * (uint32_t)a.t.slots;
     const long long n = a.n;
     for (unsigned ft = blockIdx.x; ft < a.num_wide; ft += gridDim.x) {
@@ -205,6 +206,7 @@ __global__ void __launch_bounds__(LX_THREADS, 5) lex3_write_kernel(Lex3Args a, L
     uint16_t* s_slot = reinterpret_cast<uint16_t*>(smem) + warp * LW_WARP;
     uint32_t* s_cur = reinterpret_cast<uint32_t*>(smem + 2 * NW * LW_WARP) + warp * 64;
     if (tid < S) s_tok[tid] = a.t.tokinfo[tid];
+    after_prior_kernel();
     const long long n = a.n;
     const long long ND = sg.n_docs;
     // document holding position p of this tile: the largest d in [d0, dmax]

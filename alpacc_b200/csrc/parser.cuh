@@ -392,14 +392,15 @@ __global__ void __launch_bounds__(PP_THREADS, 3) parse_pairs_kernel(ParseArgs a)
     __shared__ uint32_t s_pow[17];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int q = QT > 0 ? QT : a.t.q, k = KT > 0 ? KT : a.t.k, W = q + k;
-    if (a.dL) a.L = *a.dL;
-    if ((long long)blockIdx.x * PP_TILE >= a.L) return;  // with dL the grid covers the capacity
     for (int i = tid; i < a.t.n_pairs * (int)(sizeof(PairInfo) / 4); i += PP_THREADS)
         reinterpret_cast<uint32_t*>(s_pi)[i] = reinterpret_cast<const uint32_t*>(a.t.pairs)[i];
     if (tid == 0) {
         uint32_t pw = 1;
         for (int j = 0; j < W; ++j) { s_pow[W - 1 - j] = pw; pw *= (uint32_t)a.t.T; }
     }
+    after_prior_kernel();
+    if (a.dL) a.L = *a.dL;
+    if ((long long)blockIdx.x * PP_TILE >= a.L) return;  // with dL the grid covers the capacity
     const long long n_tiles = (a.L + PP_TILE - 1) / PP_TILE;
     // The window of a tile, one tile ahead in registers (its loads in flight while the
     // block works on the tile before): this thread's four terminals, and for the first
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(PP_THREADS, 3) parse_pairs_kernel(ParseArgs a)
     auto window_loads = [&](long long b, uint2& t4, uint32_t& te) {
         const long long i0 = b + (long long)tid * PP_ITEMS;
         if (i0 >= 0 && i0 + PP_ITEMS <= a.L && (reinterpret_cast<uintptr_t>(a.P) & 7) == 0) {
-            t4 = __ldg(reinterpret_cast<const uint2*>(a.P + i0));
+            t4 = *reinterpret_cast<const uint2*>(a.P + i0);
         } else {
             t4 = make_uint2(pos_term(a, i0) | (pos_term(a, i0 + 1) << 16), pos_term(a, i0 + 2) | (pos_term(a, i0 + 3) << 16));
         }
@@ -598,6 +599,7 @@ __global__ void __launch_bounds__(ST_CHUNK) scan_tiles_kernel(PosSums* s, long l
     __shared__ PosSums s_carry;
     __shared__ uint32_t s_chunk;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    after_prior_kernel();
     if (dL) tiles = (*dL + PP_TILE - 1) / PP_TILE;  // the grid covers the capacity
     const long long last = (tiles + ST_CHUNK - 1) / ST_CHUNK - 1;
     if (tid == 0) s_chunk = gridDim.x > 1 ? atomicAdd(sy.ticket, 1u) : 0u;

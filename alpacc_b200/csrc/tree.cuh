@@ -271,11 +271,12 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_tree_kernel(TreeArgs a) {
     __shared__ uint32_t s_en;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = PP_THREADS / 32;
-    if (a.dL) a.L = *a.dL;
-    if ((long long)blockIdx.x * PP_TILE >= a.L) return;  // with dL the grid covers the capacity
     for (int i = tid; i <= a.t.n_pairs; i += PP_THREADS) s_pr[i] = a.t.pairs[i];
     for (int i = tid; i < a.t.n_pseq; i += PP_THREADS) s_rec[i] = a.t.rec[i];
     for (int i = tid; i < a.t.n_stack; i += PP_THREADS) s_se[i] = a.t.stack[i];
+    after_prior_kernel();
+    if (a.dL) a.L = *a.dL;
+    if ((long long)blockIdx.x * PP_TILE >= a.L) return;  // with dL the grid covers the capacity
     const uint32_t NP = (uint32_t)a.t.n_pairs, last_se = (uint32_t)a.t.n_stack - 1u;
     const long long n_tiles = (a.L + PP_TILE - 1) / PP_TILE;
     // this thread's pair ids (and terminals), one tile ahead
@@ -750,6 +751,7 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_tree_kernel(TreeArgs a) {
 
 // Minima of the tiles' least D over 32 and 1024 tiles, as tile_min_levels_kernel.
 __global__ void tree_levels_kernel(TreeArgs a, long long tiles) {
+    after_prior_kernel();
     if (a.dL) tiles = min(tiles, (*a.dL + PP_TILE - 1) / PP_TILE);
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int32_t m = INT32_MAX;
@@ -757,7 +759,7 @@ __global__ void tree_levels_kernel(TreeArgs a, long long tiles) {
 #pragma unroll 8
         for (int k = 0; k < 32; ++k) {
             const long long t = g * 32 + k;
-            if (t < tiles) m = min(m, __ldg(&a.tile_min[t]));
+            if (t < tiles) m = min(m, a.tile_min[t]);
         }
         a.m32[g] = m;
     }
@@ -768,6 +770,7 @@ __global__ void tree_levels_kernel(TreeArgs a, long long tiles) {
 // The searches that left their tile, a warp per tile: the nearest earlier tile with a
 // small enough minimum, then the last small enough entry of its staircase.
 __global__ void __launch_bounds__(256) tree_escape_kernel(TreeArgs a, long long tiles) {
+    after_prior_kernel();
     if (a.dL) tiles = min(tiles, (*a.dL + PP_TILE - 1) / PP_TILE);
     const int lane = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * (blockDim.x / 32);
