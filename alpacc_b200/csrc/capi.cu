@@ -22,6 +22,7 @@
 #include "lex3.cuh"
 #include "lexwalk.cuh"
 #include "parser.cuh"
+#include "keys.cuh"
 #include "tree.cuh"
 #include "mlp.cuh"
 #include "spec.cuh"
@@ -91,6 +92,8 @@ struct alp_ctx {
     bool has_parser = false;
     ParseTables pt{};
     ParseHost ph{};
+    bool keys = false;       // parse_keys_kernel's tables fit this grammar
+    KeyTables kt{};
     bool tree = false;                    // the grammar fits parse_tree_kernel's compact tables
     TreeTables tt{};
     // ---- memory ----
@@ -1186,16 +1189,28 @@ int position_sums(alp_ctx* ctx, ParseArgs& a, ScanSync sy, long long nd) {
     a.pid = (uint16_t*)ctx->tmp[T_PID].p;
     a.tile_sums = (PosSums*)ctx->tmp[T_TSUMS].p;
     sy.sums = a.tile_sums + tiles;
-    const void* fn = pairs_kernel_for(ctx->pt.q, ctx->pt.k);
-    const size_t sm = pairs_smem_bytes(ctx->pt.n_pairs, ctx->pt.q + ctx->pt.k);
-    if ((rc = fit_blocks(ctx, fn, PP_THREADS, sm, false, &per1))) return rc;
-    const long long x = (long long)persistent_ctas(per1, ctx->tune.pairs_ctas) * ctx->sms;
-    mark(ctx, "start");
-    {
+    // (the tree kernel does not read the sums of arities, which parse_keys_kernel leaves out)
+    if (ctx->keys && !a.shard) {
+        KeyArgs ka{ctx->kt, a.P, a.pid, a.tile_sums, a.L, a.dL, (uint32_t)ctx->pt.T, ctx->pt.empty};
+        const void* fn = keys_kernel_for(ctx->pt.q, ctx->pt.k);
+        const size_t sm = keys_smem_bytes(ctx->kt.n_rec, ctx->kt.n_row, ctx->kt.n_col);
+        if ((rc = fit_blocks(ctx, fn, KW_THREADS, sm, false, &per1))) return rc;
+        // (a tuned CTA is one of parse_pairs_kernel's: two of these)
+        const long long x = (long long)persistent_ctas(per1, 2 * ctx->tune.pairs_ctas) * ctx->sms;
+        mark(ctx, "start");
+        void* args[] = {&ka};
+        if ((rc = launch_next(ctx, fn, (unsigned)(x < tiles ? x : tiles), KW_THREADS, sm, args))) return rc;
+        mark(ctx, "parse_keys_kernel");
+    } else {
+        const void* fn = pairs_kernel_for(ctx->pt.q, ctx->pt.k);
+        const size_t sm = pairs_smem_bytes(ctx->pt.n_pairs, ctx->pt.q + ctx->pt.k);
+        if ((rc = fit_blocks(ctx, fn, PP_THREADS, sm, false, &per1))) return rc;
+        const long long x = (long long)persistent_ctas(per1, ctx->tune.pairs_ctas) * ctx->sms;
+        mark(ctx, "start");
         void* args[] = {&a};
         if ((rc = launch_next(ctx, fn, (unsigned)(x < tiles ? x : tiles), PP_THREADS, sm, args))) return rc;
+        mark(ctx, "parse_pairs_kernel");
     }
-    mark(ctx, "parse_pairs_kernel");
     {
         long long t = tiles, n = nd;
         void* args[] = {&a.tile_sums, &t, &sy, &a.res, &a.node_off, &a.br_off, &n, &a.dL};
@@ -1823,6 +1838,24 @@ inline unsigned grid_for(long long n) {
     return (unsigned)(g < 1 ? 1 : g);
 }
 
+// The window tables of parse_keys_kernel, where the grammar fits them.
+int load_keys(alp_ctx* ctx) {
+    KeyHost h;
+    if (!build_key_tables(ctx->ph, h)) return ALP_OK;
+    KeyTables& t = ctx->kt;
+    t.n_row = (int)h.row.size();
+    t.n_col = (int)h.col.size();
+    t.n_rec = (int)(h.rec.size() / 2);
+    const uint32_t* rec;
+    int rc;
+    if ((rc = upload(ctx, h.row.data(), h.row.size(), &t.row)) || (rc = upload(ctx, h.col.data(), h.col.size(), &t.col)) ||
+        (rc = upload(ctx, h.rec.data(), h.rec.size(), &rec)))
+        return rc;
+    t.rec = reinterpret_cast<const uint2*>(rec);
+    ctx->keys = true;
+    return ALP_OK;
+}
+
 // The compact tables of parse_tree_kernel, where the grammar fits them.
 int load_tree(alp_ctx* ctx) {
     TreeHost h;
@@ -1957,6 +1990,7 @@ int alp_ctx_create(const void* blob, size_t len, int device, alp_ctx** out) {
     if (!rc && hp) rc = load_parser(ctx->pt, ctx->ph, r.p, r.e, ctx->owned, ctx->err);
     if (!rc && hp) ctx->has_parser = true;
     if (!rc && hp) rc = load_tree(ctx);
+    if (!rc && hp && ctx->tree) rc = load_keys(ctx);
     if (!rc && hl && hp) {
         // the parser indexes its key table with the lexer's terminal ids
         const uint32_t T = (uint32_t)ctx->pt.T;
@@ -2213,6 +2247,12 @@ int alp_tune_parse(alp_ctx* ctx, const uint8_t* d_in, int64_t n, int reps, char*
         if ((rc = fit_blocks(ctx, pairs_kernel_for(ctx->pt.q, ctx->pt.k), PP_THREADS, sm1, false, &fit_pairs)) ||
             (rc = fit_blocks(ctx, ex, PP_THREADS, sm2, false, &fit_expand)))
             return done(rc);
+        if (ctx->keys) {
+            if ((rc = fit_blocks(ctx, keys_kernel_for(ctx->pt.q, ctx->pt.k), KW_THREADS,
+                                 keys_smem_bytes(ctx->kt.n_rec, ctx->kt.n_row, ctx->kt.n_col), false, &fit_pairs)))
+                return done(rc);
+            fit_pairs = (fit_pairs + 1) / 2;
+        }
     }
     best = 1e30;
     arg = 0;
@@ -4156,6 +4196,8 @@ alp_ctx* child_ctx(const alp_ctx* p) {
     c->pt = p->pt;
     c->ph = p->ph;
     c->tree = p->tree;
+    c->keys = p->keys;
+    c->kt = p->kt;
     c->tt = p->tt;
     c->tune = p->tune;
     return c;

@@ -310,7 +310,7 @@ __device__ __forceinline__ PosSums ps_warp_scan(PosSums x, int lane) {
 // rights, then its lefts, so position p's first rights close position p-1's
 // top lefts, min(lefts of p-1, rights of p) of them, unless p starts a
 // document or either has no pair.
-__device__ __forceinline__ uint32_t pair_lefts(const PairInfo& p) {
+__host__ __device__ __forceinline__ uint32_t pair_lefts(const PairInfo& p) {
     return (uint32_t)(((int32_t)p.n_br + (int32_t)p.d_depth) >> 1);
 }
 __device__ __forceinline__ uint32_t adj_closed(const PairInfo* s_pi, uint32_t prev, uint32_t cur, bool head) {

@@ -348,6 +348,7 @@ def _kernel_alg_bytes(name, units, parse_layout=True):
         "lex3_write_kernel": 2 * c + 2 * m + tok * m,          # chunk counts and token records in, tokens out
         "lex3_fold_kernel": n + c,                             # bytes in, an endomorphism per 64 bytes out
         "lex3_walk_kernel": n + c // 2 + 3 * c + 2 * m,        # bytes, states in, chunk states, counts and records out
+        "parse_keys_kernel": 4 * L,                            # terminal ids in, pair ids out
         "parse_pairs_kernel": 4 * L,                           # terminal ids in, pair ids out
     }
     return table.get(name)
