@@ -1354,15 +1354,18 @@ int run_tree_escapes(alp_ctx* ctx, TreeArgs& t) {
     const long long tiles = (t.L + PP_TILE - 1) / PP_TILE;
     mark(ctx, "start");
     long long count = tiles;
-    void* args[] = {&t, &count};
-    int rc;
-    // up to 32 tiles, the tiles' own minima are one group: no search goes above them
-    if (tiles > 32 && (rc = launch_next(ctx, (const void*)tree_levels_kernel, (unsigned)(((tiles + 31) / 32 + 255) / 256), 256,
-                                        0, args)))
+    int rc, split = tiles <= TR_LEVELS ? 8 : 1;
+    void* args[] = {&t, &count, &split};
+    // Up to 1024 tiles (some 2 M positions) the searches read the one block's minima
+    // themselves, 4 KB a warp, and a tile has eight warps: without the launch of the levels and
+    // with more searches at once 4 MB of json take 133 us, not 139.
+    const bool levels = tiles > TR_LEVELS;
+    if (levels && (rc = launch_next(ctx, (const void*)tree_levels_kernel, (unsigned)(((tiles + 31) / 32 + 255) / 256), 256, 0,
+                                    args)))
         return rc;
-    const long long g = (tiles + 7) / 8;
+    const long long g = (tiles * split + 7) / 8;
     if ((rc = launch_next(ctx, (const void*)tree_escape_kernel, (unsigned)(g < 148 * 8 ? g : 148 * 8), 256, 0, args))) return rc;
-    mark(ctx, "tree_levels+tree_escape");
+    mark(ctx, levels ? "tree_levels+tree_escape" : "tree_escape_kernel");
     return ALP_OK;
 }
 

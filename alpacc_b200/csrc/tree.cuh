@@ -772,6 +772,7 @@ __global__ void tree_levels_kernel(TreeArgs a, long long tiles) {
 // 1024-block, so that only a search that goes further reads memory step by step (each step
 // some 500 cycles: a walk over a group took up to 8 us).  In a group found further off, 32
 // minima are read at once.
+constexpr long long TR_LEVELS = 1024;  // up to these tiles tree_escape_kernel needs no levels
 __device__ __forceinline__ long long tr_last_leq(const int32_t* v, int32_t d) {
     int at = -1;
 #pragma unroll
@@ -796,27 +797,43 @@ __device__ __forceinline__ long long tr_prev_tile(const TreeArgs& a, const int32
     return g * 32 + tr_last_leq(a.tile_min + g * 32, d);
 }
 
-// The searches that left their tile, a warp per tile: the nearest earlier tile with a
-// small enough minimum, then the last small enough entry of its staircase.
+// The searches that left their tile, `split` warps a tile (1 or 8): the nearest earlier tile
+// with a small enough minimum, then the last small enough entry of its staircase.  A search is
+// some ten dependent loads, so few tiles are spread over the SMs eight warps each.
 // With the minima staged so, 22 -> 17 us at 4 MB of json (of it 6 for the two launches); 38 us
 // at 256 MiB as before.
-__global__ void __launch_bounds__(256) tree_escape_kernel(TreeArgs a, long long tiles) {
+__global__ void __launch_bounds__(256) tree_escape_kernel(TreeArgs a, long long tiles, int split) {
     __shared__ int32_t s_min[8][32], s_m32[8][32];
     after_prior_kernel();
     if (a.dL) tiles = min(tiles, (*a.dL + PP_TILE - 1) / PP_TILE);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long warps = (long long)gridDim.x * (blockDim.x / 32);
-    for (long long t = (long long)blockIdx.x * (blockDim.x / 32) + warp; t < tiles; t += warps) {
+    for (long long wt = (long long)blockIdx.x * (blockDim.x / 32) + warp; wt < tiles * split; wt += warps) {
+        const long long t = wt / split;
+        const uint32_t first = (uint32_t)(wt % split) * 32u;
         const TreeTile tt = a.tiles[t];
-        if (tt.esc == 0) continue;
+        if (tt.esc <= first) continue;
         {
             const long long u = (t & ~31ll) + lane, g = ((t >> 5) & ~31ll) + lane;
             __syncwarp();
             s_min[warp][lane] = u < t ? a.tile_min[u] : INT32_MAX;
-            s_m32[warp][lane] = g < (t >> 5) ? a.m32[g] : INT32_MAX;
+            int32_t m = INT32_MAX;
+            if (g < (t >> 5)) {
+                if (tiles > TR_LEVELS) {
+                    m = a.m32[g];
+                } else {  // no level was built: a lane reads its group of the one block
+                    const int4* v = reinterpret_cast<const int4*>(a.tile_min + g * 32);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int4 x = v[k];
+                        m = min(m, min(min(x.x, x.y), min(x.z, x.w)));
+                    }
+                }
+            }
+            s_m32[warp][lane] = m;
             __syncwarp();
         }
-        for (uint32_t e = lane; e < tt.esc; e += 32) {
+        for (uint32_t e = first + lane; e < tt.esc; e += 32u * (uint32_t)split) {
             const uint2 q = a.esc[(size_t)tt.node_base + t + e];
             const int32_t d = (int32_t)q.x;
             const long long pos = t * PP_TILE + (q.y & 2047u);
@@ -829,6 +846,14 @@ __global__ void __launch_bounds__(256) tree_escape_kernel(TreeArgs a, long long 
                 const TreeTile tu = a.tiles[u];
                 const uint2* sv = a.stair + (size_t)u * PP_TILE;
                 int lo = 0, hi = (int)tu.stair - 1;  // the last entry <= d (they ascend)
+                while (hi - lo >= 4) {  // three probes at a time: a round is one trip to memory
+                    const int s4 = (hi - lo) >> 2, p1 = lo + s4, p2 = p1 + s4, p3 = p2 + s4;
+                    const bool b1 = (int32_t)sv[p1].x <= d, b2 = (int32_t)sv[p2].x <= d, b3 = (int32_t)sv[p3].x <= d;
+                    if (!b1) hi = p1 - 1;
+                    else if (!b2) { lo = p1; hi = p2 - 1; }
+                    else if (!b3) { lo = p2; hi = p3 - 1; }
+                    else lo = p3;
+                }
                 while (lo < hi) {
                     const int mid = (lo + hi + 1) >> 1;
                     if ((int32_t)sv[mid].x <= d) lo = mid; else hi = mid - 1;
