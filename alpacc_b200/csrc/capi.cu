@@ -2682,8 +2682,8 @@ static int stream_piece(alp_ctx* ctx, LexCarry* carry, const uint8_t* d_in, long
     r.a.carry_tokens = global;
     r.a.tok_first = first;
     if ((rc = lex3_front(ctx, r)) || (rc = lex3_emit<uint32_t, int64_t>(ctx, r))) return rc;
-    lex3_stream_tail_kernel<<<1, LX_THREADS, 0, ctx->stream>>>(r.a);
-    CK(cudaGetLastError());
+    void* args[] = {&r.a};
+    if ((rc = launch_next(ctx, (const void*)lex3_stream_tail_kernel, 1, LX_THREADS, 0, args))) return rc;
     mark(ctx, "lex3_stream_tail_kernel");
     return ALP_OK;
 }
@@ -4068,6 +4068,7 @@ namespace {
 // counts[0] nodes, [1] brackets, [2] positions, [3] ALP_DEV_ERR_* bits
 __global__ void batch_status_kernel(const AlpResult* lex, const AlpResult* res, long long cap_nodes, long long cap_brs,
                                     long long* counts) {
+    after_prior_kernel();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     unsigned int err = res->error | lex->error;
     if (res->aux[0] > cap_nodes || res->aux[1] > cap_brs) err |= ALP_DEV_ERR_CAPACITY;
@@ -4177,9 +4178,10 @@ int graph_enqueue(alp_parse_graph* g) {
     if ((rc = parse_positions_dev(ctx, n + 2 * nd, &r.a.res->aux[5], nd, g->d_valid, g->o, g->cap_nodes, g->cap_brs,
                                   (long long*)g->d_node_off, d_res, r.pos_sync)))
         return rc;
-    batch_status_kernel<<<1, 32, 0, ctx->stream>>>(r.a.res, d_res, g->cap_nodes, g->cap_brs, (long long*)g->d_counts);
-    CK(cudaGetLastError());
-    return ALP_OK;
+    const AlpResult *lex = r.a.res, *res = d_res;
+    long long* counts = (long long*)g->d_counts;
+    void* args[] = {&lex, &res, &g->cap_nodes, &g->cap_brs, &counts};
+    return launch_next(ctx, (const void*)batch_status_kernel, 1, 32, 0, args);
 }
 
 alp_ctx* child_ctx(const alp_ctx* p) {

@@ -1212,6 +1212,25 @@ __global__ void __launch_bounds__(LX_THREADS) lex3_stream_tail_kernel(Lex3Args a
     __shared__ long long s_best[LX_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long C = a.n_chunks, T = a.num_tiles;
+    after_prior_kernel();
+    // The state after the last chunk, in warp 0: lane s reads what each byte makes of state s,
+    // all loads at once, and the chunk's state is followed through them by shuffles (one load
+    // after another took 8 us).
+    uint32_t st = 0;
+    if (warp == 0) {
+        const long long p0 = (C - 1) * LX_CHUNK;
+        const int lim = (int)(a.n - p0);
+        const uint32_t mine = lane < lim ? a.in[p0 + lane] : 0u;
+        uint32_t to[LX_CHUNK];
+#pragma unroll
+        for (int j = 0; j < LX_CHUNK; ++j) {
+            const uint32_t b = __shfl_sync(ALP_FULL_MASK, mine, j);
+            to[j] = (j < lim && lane < a.t.S) ? (uint32_t)(a.t.ent[lane * LX_ROW + b] & LX_NEXT) : (uint32_t)lane;
+        }
+        st = a.chunk_s[C - 1] & 31u;
+#pragma unroll
+        for (int j = 0; j < LX_CHUNK; ++j) st = __shfl_sync(ALP_FULL_MASK, to[j], st & 31u);
+    }
     long long best = -1;  // last token start in the last tile
     for (long long c = (T - 1) * (LX_TILE / LX_CHUNK) + tid; c < C; c += LX_THREADS) {
         const uint32_t off = a.chunk_c[c] >> 8;
@@ -1229,8 +1248,6 @@ __global__ void __launch_bounds__(LX_THREADS) lex3_stream_tail_kernel(Lex3Args a
         }
         LexCarry* c = a.carry;
         if (best >= 0) c->start = a.pos_base + best;
-        uint32_t st = a.chunk_s[C - 1];
-        for (long long p = (C - 1) * LX_CHUNK; p < a.n; ++p) st = a.t.ent[st * LX_ROW + a.in[p]] & LX_NEXT;
         c->state = st;
         c->piece = a.res->count;
         c->tokens += a.res->count;
