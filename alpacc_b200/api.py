@@ -445,7 +445,7 @@ class Grammar:
 
     def get_tuning(self) -> List[int]:
         """[tile shape, pair CTAs per SM, expand CTAs per SM, MLP kernel (0 tcgen05, 1 mma.sync),
-        lexer token pass (0 fused, 1 count pass + tile scan + token pass),
+        lexer token pass (0 fused, 1 walk with token records + tile scan + write pass),
         parser position pass (0 fused, 1 pair pass + tile-sum scan + expansion),
         lexer state-scan chunks per lane (8, 16 or 32)]."""
         cfg = (ctypes.c_int32 * 7)()

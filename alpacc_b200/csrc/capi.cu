@@ -69,9 +69,9 @@ struct Tuning {
     int pairs_ctas = 0;   // CTAs per SM of the persistent pair kernel (0: as many as fit)
     int expand_ctas = 0;  // same for the expand kernel
     int mlp = 0;          // boundary-MLP inference: 0 tcgen05 kernel, 1 mma.sync kernel
-    int lex_split = 1;    // lexer token pass: 0 fused (counts, look-back, tokens), 1 count pass + tile scan + token pass
+    int lex_split = 1;    // lexer token pass: 0 fused (counts, look-back, tokens), 1 walk + tile scan + write
     int parse_split = 1;  // parser position pass: 0 fused (pairs, look-back, expand), 1 pair pass + scan + expand
-    int scan_g = 0;       // lexer state scan: chunks per lane, 8, 16 or 32 (0: LS_G)
+    int scan_g = 0;       // lexer state scan: units per lane, 8, 16 or 32 (0: LS_G)
 };
 
 struct alp_ctx {

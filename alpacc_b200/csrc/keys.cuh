@@ -5,19 +5,20 @@
 // cut at its document's ⊢ and ⊣.  The cut is in the tables: the window as it stands in memory
 // is split into a left part (up to the position's own terminal) and a right part, each with a
 // number for its class (left parts with the same pairs under every right part, and the other
-// way round: json's 225 x 225 windows are some hundred records), and the record at (left
-// class, right class) holds all that the pair adds up to, its id and whether the position is
-// a ⊢.  So a position costs one or two 16-bit and one 8-byte load from shared memory, no
+// way round: json's 225 x 225 windows are 63 x 56 records, sexp's 49 are 16), and the record
+// at (left class, right class) holds all that the pair adds up to, its id and whether the
+// position is a ⊢.  So a position costs one or two 16-bit and one 8-byte load from shared memory, no
 // comparison with the sentinels and no load from a key table in global memory.
 //
 // A warp takes a tile by itself, 8 positions a lane at a time, so there is no barrier: the
 // terminals next to a lane's come from its neighbours by shuffles, and sums of up to 31 a
 // position (the compact tables' limit) are added as bytes, four fields a word.  The eight
 // positions with a ⊢ among them (rare but for batches of tiny documents) take the segmented
-// sums.  Memory traffic is 4 B a position (50 us of the figures below).
+// sums.  Memory traffic is 4 B a position.
 //
-// At 256 MiB of json (82 M positions) 230 -> 70 us against parse_pairs_kernel, 38 -> 18 us at
-// 32 MB, in batches of 13 KB documents 232 -> 72; up to 4 MB both are launch and latency, 12 us.
+// At 256 MiB of json (37.5 M positions, 23 us of traffic at the measured copy rate) 230 -> 70
+// us against parse_pairs_kernel, 38 -> 18 us at 32 MB, in batches of 13 KB documents 232 ->
+// 72; up to 4 MB both are launch and latency, 12 us.
 // The shared-memory pipe bounds it: two loads a position with a few lanes on one bank.
 #pragma once
 

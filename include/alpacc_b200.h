@@ -91,8 +91,8 @@ int alp_check_bounded_wait(alp_ctx* ctx);
  * (0: tcgen05 tensor-memory kernel, the default; 1: mma.sync kernel, whose
  * predictions may differ where two logits are within rounding); with n >= 5,
  * cfg[4] the lexer's token pass (0: one fused pass that counts, looks back
- * over tiles and writes tokens; 1: a count pass, a tile scan and a token
- * pass, the default); with n >= 6, cfg[5] the parser's position pass (0: one
+ * over tiles and writes tokens; 1: a walk that counts and records tokens, a
+ * tile scan and a write pass, the default); with n >= 6, cfg[5] the parser's position pass (0: one
  * fused pass that looks up the pairs, looks back over tiles and expands, sized
  * from the previous parse on the context; 1: a pair pass and a scan of its
  * tile sums before the expansion, the default); with n >= 7, cfg[6] the lexer state
