@@ -52,6 +52,15 @@ constexpr uint32_t TR_END = 0xfeu;
 constexpr uint32_t TR_NO_NODE = 0xffffu;  // a listed search: no node takes its answer
 constexpr int TR_NONE = INT32_MAX;
 
+// Whether a search that its tile cannot answer is listed for tree_escape_kernel: the right
+// leaves depth d, `node` is the node that takes the answer, or TR_NO_NODE.  A tile's list has
+// room for its nodes and one more.  Entries with a node pay for themselves.  Without one there
+// is only the ⊣ that pops the end marker: from depth 0 or more its left lies in its own
+// document, so only the document that the tile continues lists it, once; below depth 0 no left
+// can match and the position has rejected its document already.  (A batch of documents such
+// as json's `1 2`, no pair but ⊣'s, would list hundreds a tile where there are no nodes.)
+__host__ __device__ inline bool tr_listed(int32_t d, uint32_t node) { return d >= 0 || node != TR_NO_NODE; }
+
 struct TreeTables {
     const uint2* pairs;     // [n_pairs + 1]
     const uint2* rec;       // [n_pseq]
@@ -185,8 +194,7 @@ struct TreeArgs {
     int span_cap;
     // searches that leave a tile
     // depth; position in the tile | right << 11 | tile-local node << 16.  A tile's list has
-    // room for its nodes and one more (a ⊣ pops the end marker for no node): it starts at
-    // its first node + its number
+    // room for its nodes and one more (tr_listed): it starts at its first node + its number
     uint2* esc;                 // [esc_cap], cap_nodes + tiles
     long long esc_cap;
     uint2* stair;               // [tiles * PP_TILE] D; position in the tile | first node (tile-local) << 16
@@ -681,7 +689,7 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_tree_kernel(TreeArgs a) {
                             const uint32_t p = match(at, d, me, ONE ? 0u : s_hd[pl], pl);
                             if (r == 0) q[e] = p;
                             else if (a.parent && node != TR_NO_NODE && gi < a.cap_nodes) a.parent[gi] = (long long)p;
-                        } else {
+                        } else if (tr_listed(d, node)) {
                             const long long k = (long long)tp.nodes + tile + atomicAdd(&s_en, 1u);
                             if (k < a.esc_cap) a.esc[k] = make_uint2((uint32_t)d, (uint32_t)pl | (r << 11) | (node << 16));
                         }
