@@ -1020,7 +1020,9 @@ int lex3_run(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long* d_
 // The lexer API layout into buffers from the caller's allocator: the token total
 // (and one document's verdict) is known after the tile scan, before any token is
 // written, so the outputs are allocated at their exact size and the token pass
-// writes them once.  One document that is rejected gets no outputs.
+// writes them once.  accepted (one document that is no batch): its verdict; a
+// rejected one gets no outputs.  Null for a batch, of one document too: its
+// offsets and validity are written whatever the verdicts.
 int lex3_run_alloc(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long* d_off, long long nd,
                    uint8_t* valid, void** ptrs, long long* total, int* accepted) {
     Lex3Run r;
@@ -1037,7 +1039,7 @@ int lex3_run_alloc(alp_ctx* ctx, const uint8_t* d_in, long long n, const long lo
     if (ctx->h_res->error & ALP_DEV_ERR_TIMEOUT) return fail(ctx, ALP_ERR_TIMEOUT, "lexer look-back timed out");
     const long long m = ctx->h_res->aux[6];
     ctx->last_tokens = m;
-    if (nd == 1) {
+    if (accepted) {
         *accepted = ctx->h_res->aux[7] ? 1 : 0;
         if (!*accepted) return ALP_OK;
     }
@@ -3954,11 +3956,10 @@ int alp_lex_batch(alp_ctx* ctx, const uint8_t* d_in, const int64_t* d_off, int64
     if (ctx->alloc_fn && ctx->lex3 && ctx->tune.lex_split && n > 0) {
         void* p[3] = {};
         long long total = 0;
-        int accepted = 0;
         if ((rc = grow(ctx, ctx->tmp[T_DVALID], (size_t)n_docs + 16)) ||
             (rc = grow(ctx, ctx->tmp[T_TOKOFF], (size_t)(n_docs + 1) * 8)) ||
             (rc = lex3_run_alloc(ctx, d_in, n, (const long long*)d_off, n_docs, (uint8_t*)ctx->tmp[T_DVALID].p, p,
-                                 &total, &accepted)))
+                                 &total, nullptr)))
             return rc;
         *d_term = (uint32_t*)p[0];
         *d_start = (int64_t*)p[1];

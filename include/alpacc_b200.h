@@ -119,8 +119,8 @@ int alp_memcpy(alp_ctx* ctx, void* dst, const void* src, size_t bytes);
  * kind, start, end, of n elements each; a batch also copies its n_docs + 1
  * offsets to ptrs[ALP_ALLOC_OFF] and its validity to ptrs[ALP_ALLOC_VALID] where
  * these are set (they are null on entry).  A nonzero return ends the call with
- * ALP_ERR_CUDA.  It must not call back into the context.  An input that is
- * rejected may get no call.  fn NULL: outputs are owned by the context again. */
+ * ALP_ERR_CUDA.  It must not call back into the context.  A single input that is
+ * rejected may get no call; a batch gets one whatever its documents' verdicts.  fn NULL: outputs are owned by the context again. */
 enum { ALP_ALLOC_OFF = 5, ALP_ALLOC_VALID = 6, ALP_ALLOC_PTRS = 7 };
 typedef int (*alp_alloc_fn)(void* user, int64_t n, void** ptrs);
 int alp_set_output_alloc(alp_ctx* ctx, alp_alloc_fn fn, void* user);
