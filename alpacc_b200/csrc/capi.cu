@@ -1436,7 +1436,8 @@ bool ahead_ok(const alp_ctx* ctx, long long n, long long nd) {
     return ctx->lex3 && ctx->tune.lex_split && ctx->tune.parse_split && n > 0 && n + 2 * nd <= AHEAD_MAX;
 }
 
-// Lexer and pair sums of n bytes in one run of launches, with one wait for both results.
+// Lexer and pair sums of n bytes in one run of launches, with one wait for both results.  The
+// pair ids have the token buffer's capacity: what goes past it is the lexer's capacity error.
 // *m: tokens.  valid (one document): the lexer's verdict, and *dvalid moves into the head.
 int lex_pairs(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long* d_off, long long nd, long long tcap,
               uint8_t** dvalid, PosHead* h, long long* m, uint8_t* valid) {
@@ -1450,7 +1451,7 @@ int lex_pairs(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long* d
     h->base = r.base;
     h->sy = r.pos_sync;
     if ((rc = lex3_front(ctx, r)) || (rc = lex3_emit<uint16_t, uint32_t>(ctx, r)) ||
-        (rc = parse_args(ctx, n + 2 * nd, nd, *dvalid, 1, head_result(*h), h->a)))
+        (rc = parse_args(ctx, tcap, nd, *dvalid, 1, head_result(*h), h->a)))
         return rc;
     h->a.dL = &r.a.res->aux[5];
     AlpResult lex;
@@ -4176,7 +4177,7 @@ int graph_enqueue(alp_parse_graph* g) {
         return rc;
     // (positions of the batch: the tile scan's total in the lexer's result)
     AlpResult* d_res = reinterpret_cast<AlpResult*>(r.base + SC_PARSE);
-    if ((rc = parse_positions_dev(ctx, n + 2 * nd, &r.a.res->aux[5], nd, g->d_valid, g->o, g->cap_nodes, g->cap_brs,
+    if ((rc = parse_positions_dev(ctx, (long long)tcap, &r.a.res->aux[5], nd, g->d_valid, g->o, g->cap_nodes, g->cap_brs,
                                   (long long*)g->d_node_off, d_res, r.pos_sync)))
         return rc;
     const AlpResult *lex = r.a.res, *res = d_res;

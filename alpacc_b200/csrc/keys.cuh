@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(KW_THREADS) parse_keys_kernel(KeyArgs a) {
     for (int i = tid; i < a.t.n_row; i += KW_THREADS) s_row[i] = a.t.row[i];
     for (int i = tid; i < a.t.n_col; i += KW_THREADS) s_col[i] = a.t.col[i];
     after_prior_kernel();
-    if (a.dL) a.L = *a.dL;
+    a.L = position_count(a.L, a.dL);
     __syncthreads();
     const long long L = a.L, n_tiles = (L + PP_TILE - 1) / PP_TILE;
     const uint32_t T = a.T, EE = a.empty | (a.empty << 16);

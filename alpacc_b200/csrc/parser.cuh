@@ -367,6 +367,14 @@ struct ParseArgs {
     int span_cap;
 };
 
+// The positions of a launch sized for `cap`: their count in device memory where dL is set.  A
+// count past the capacity (a lexer that ends empty tokens can give three positions a byte) is
+// cut to it, so that no kernel leaves its buffers; the lexer's result carries the capacity
+// error, which the host reads with the counts.
+__host__ __device__ inline long long position_count(long long cap, const long long* dL) {
+    return dL && *dL < cap ? *dL : cap;
+}
+
 __device__ __forceinline__ uint32_t pos_term(const ParseArgs& a, long long i) {
     if (i < 0) return (a.shard && i >= -PS_HALO) ? __ldg(&a.halo[PS_HALO + i]) : a.t.empty;
     if (i >= a.L) return (a.shard && i - a.L < PS_HALO) ? __ldg(&a.halo[PS_HALO + (i - a.L)]) : a.t.empty;
@@ -399,7 +407,7 @@ __global__ void __launch_bounds__(PP_THREADS, 3) parse_pairs_kernel(ParseArgs a)
         for (int j = 0; j < W; ++j) { s_pow[W - 1 - j] = pw; pw *= (uint32_t)a.t.T; }
     }
     after_prior_kernel();
-    if (a.dL) a.L = *a.dL;
+    a.L = position_count(a.L, a.dL);
     if ((long long)blockIdx.x * PP_TILE >= a.L) return;  // with dL the grid covers the capacity
     const long long n_tiles = (a.L + PP_TILE - 1) / PP_TILE;
     // The window of a tile, one tile ahead in registers (its loads in flight while the
@@ -600,7 +608,7 @@ __global__ void __launch_bounds__(ST_CHUNK) scan_tiles_kernel(PosSums* s, long l
     __shared__ uint32_t s_chunk;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     after_prior_kernel();
-    if (dL) tiles = (*dL + PP_TILE - 1) / PP_TILE;  // the grid covers the capacity
+    tiles = (position_count(tiles * PP_TILE, dL) + PP_TILE - 1) / PP_TILE;  // the grid covers the capacity
     const long long last = (tiles + ST_CHUNK - 1) / ST_CHUNK - 1;
     if (tid == 0) s_chunk = gridDim.x > 1 ? atomicAdd(sy.ticket, 1u) : 0u;
     __syncthreads();
@@ -847,7 +855,7 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_expand_kernel(ParseArgs a
     __shared__ uint32_t s_pow[17];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int q = QT > 0 ? QT : a.t.q, k = KT > 0 ? KT : a.t.k, W = q + k;
-    if (a.dL) a.L = *a.dL;
+    a.L = position_count(a.L, a.dL);
     for (int i = tid; i < a.t.n_pairs * (int)(sizeof(PairInfo) / 4); i += PP_THREADS)
         reinterpret_cast<uint32_t*>(s_pi)[i] = reinterpret_cast<const uint32_t*>(a.t.pairs)[i];
     for (int i = tid; i < a.t.n_pseq; i += PP_THREADS) s_prec[i] = a.t.pseq_rec[i];

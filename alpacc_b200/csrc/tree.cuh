@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_tree_kernel(TreeArgs a) {
     for (int i = tid; i < a.t.n_pseq; i += PP_THREADS) s_rec[i] = a.t.rec[i];
     for (int i = tid; i < a.t.n_stack; i += PP_THREADS) s_se[i] = a.t.stack[i];
     after_prior_kernel();
-    if (a.dL) a.L = *a.dL;
+    a.L = position_count(a.L, a.dL);
     if ((long long)blockIdx.x * PP_TILE >= a.L) return;  // with dL the grid covers the capacity
     const uint32_t NP = (uint32_t)a.t.n_pairs, last_se = (uint32_t)a.t.n_stack - 1u;
     const long long n_tiles = (a.L + PP_TILE - 1) / PP_TILE;
@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(PP_THREADS, 2) parse_tree_kernel(TreeArgs a) {
 // Minima of the tiles' least D over 32 and 1024 tiles, as tile_min_levels_kernel.
 __global__ void tree_levels_kernel(TreeArgs a, long long tiles) {
     after_prior_kernel();
-    if (a.dL) tiles = min(tiles, (*a.dL + PP_TILE - 1) / PP_TILE);
+    tiles = (position_count(tiles * PP_TILE, a.dL) + PP_TILE - 1) / PP_TILE;
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int32_t m = INT32_MAX;
     if (g < (tiles + 31) / 32) {
@@ -813,7 +813,7 @@ __device__ __forceinline__ long long tr_prev_tile(const TreeArgs& a, const int32
 __global__ void __launch_bounds__(256) tree_escape_kernel(TreeArgs a, long long tiles, int split) {
     __shared__ int32_t s_min[8][32], s_m32[8][32];
     after_prior_kernel();
-    if (a.dL) tiles = min(tiles, (*a.dL + PP_TILE - 1) / PP_TILE);
+    tiles = (position_count(tiles * PP_TILE, a.dL) + PP_TILE - 1) / PP_TILE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long warps = (long long)gridDim.x * (blockDim.x / 32);
     for (long long wt = (long long)blockIdx.x * (blockDim.x / 32) + warp; wt < tiles * split; wt += warps) {
