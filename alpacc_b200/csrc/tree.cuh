@@ -133,7 +133,8 @@ inline bool build_tree_tables(const std::vector<PairInfo>& info, const std::vect
                 ++taken;
                 right_node.push_back((uint32_t)k);
             }
-            for (int c = 0; c < arity[pseq[j]]; ++c) open.push_back((uint32_t)k);
+            // (past 15 lefts and a pop by each of 31 nodes the ends cannot become the lefts any more)
+            for (int c = 0; c < arity[pseq[j]] && open.size() < 64; ++c) open.push_back((uint32_t)k);
             // pairs of different positions may share records: they must agree
             const uint32_t y = (uint32_t)terms | (code << 24);
             if (h.rec[2 * j + 1] && h.rec[2 * j + 1] != y) return false;
