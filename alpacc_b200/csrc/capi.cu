@@ -1787,7 +1787,8 @@ int tokens_in(alp_ctx* ctx, const uint32_t* term, const int64_t* ts, const int64
     const long long g = (m + 2 + 255) / 256;
     tokens_in_kernel<<<(unsigned)(g < 148 * 8 ? g : 148 * 8), 256, 0, ctx->stream>>>(
         term, ts, te, m, (uint16_t*)ctx->tmp[T_TTERM].p, (uint32_t*)ctx->tmp[T_TSTART].p, (uint32_t*)ctx->tmp[T_TEND].p,
-        ctx->pt.start, ctx->pt.end, (uint32_t)ctx->pt.T, ctx->pt.empty, lex, h->base + SC_VALID);
+        ctx->pt.start, ctx->pt.end, (uint32_t)ctx->pt.T, std::min(ctx->pt.empty, (uint32_t)ctx->pt.T - 1u), lex,
+        h->base + SC_VALID);
     CK(cudaGetLastError());
     if (!ctx->tune.parse_split) {
         AlpResult ids;

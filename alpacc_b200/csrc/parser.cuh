@@ -86,6 +86,12 @@ inline int load_parser(ParseTables& pt, ParseHost& ph, const uint8_t* p, const u
         err = "parser tables out of range";
         return 4;
     }
+    // the key tables are indexed with them: ⊢ and ⊣ at every document's ends, the empty symbol
+    // where a window reaches past them
+    if (start >= T || end >= T || (empty >= T && q + k > 1)) {
+        err = "parser sentinel ids out of range";
+        return 4;
+    }
     auto need = [&](size_t bytes) { return p + bytes <= e; };
     if (!need((size_t)n_prods * 8)) { err = "truncated arities"; return 4; }
     std::vector<int32_t> arity(n_prods), pterm(n_prods);

@@ -20,10 +20,39 @@ static bool arity(int32_t children) {
     return build_tree_tables(info, use, stack, pseq, {children}, {-1}, h);
 }
 
+// The parser section of a blob with two terminals and the sentinels given; no pairs, no keys.
+static std::vector<uint8_t> section(uint32_t q, uint32_t k, uint32_t T, uint32_t empty, uint32_t start, uint32_t end,
+                                    const std::vector<uint32_t>& pseq = {}) {
+    std::vector<uint32_t> w = {q, k, T, empty, start, end, 1, 2, 0, 0xffffffffu, 0, 0, (uint32_t)pseq.size()};
+    w.insert(w.end(), pseq.begin(), pseq.end());
+    w.push_back(0);
+    std::vector<uint8_t> b(4 * w.size());
+    memcpy(b.data(), w.data(), b.size());
+    return b;
+}
+
+// load_parser's refusal, or "" where it got as far as the uploads (which fail without a device)
+static std::string refusal(const std::vector<uint8_t>& b) {
+    ParseTables pt{};
+    ParseHost ph;
+    std::vector<void*> owned;
+    std::string err;
+    load_parser(pt, ph, b.data(), b.data() + b.size(), owned, err);
+    return err.compare(0, 10, "cudaMalloc") == 0 ? "" : err;
+}
+
+static bool sentinels() {
+    const std::string no = "parser sentinel ids out of range";
+    return refusal(section(1, 1, 5, 2, 3, 4)).empty() && refusal(section(0, 1, 5, 5, 3, 4)).empty() &&
+           refusal(section(1, 1, 5, 5, 3, 4)) == no && refusal(section(1, 3, 5, 0x7fffffffu, 3, 4)) == no &&
+           refusal(section(1, 1, 5, 2, 5, 4)) == no && refusal(section(0, 1, 5, 2, 3, 0x40000000u)) == no;
+}
+
 int main(int argc, char** argv) {
     const char* name = argc > 1 ? argv[1] : "";
     bool ok = false;
     if (!strcmp(name, "arity")) ok = arity(0) && !arity(1) && !arity(64) && !arity(INT32_MAX);
+    if (!strcmp(name, "sentinels")) ok = sentinels();
     if (ok) printf("ok\n");
     return ok ? 0 : 1;
 }
