@@ -109,6 +109,9 @@ inline int load_parser(ParseTables& pt, ParseHost& ph, const uint8_t* p, const u
     if (!u32(n_pseq) || !need((size_t)n_pseq * 4)) { err = "bad productions"; return 4; }
     std::vector<uint32_t> pseq(n_pseq);
     memcpy(pseq.data(), p, 4 * (size_t)n_pseq); p += 4 * (size_t)n_pseq;
+    // (all of them, not only those of a pair: the records below are made for each)
+    for (uint32_t v : pseq)
+        if (v >= n_prods) { err = "production id out of range"; return 4; }
     uint32_t n_keys;
     const uint32_t W = q + k;
     if (!u32(n_keys) || !need((size_t)n_keys * (W + 1) * 4)) { err = "bad keys"; return 4; }
@@ -150,7 +153,6 @@ inline int load_parser(ParseTables& pt, ParseHost& ph, const uint8_t* p, const u
         int dd = 0, dv = 0, nt = 0;
         for (uint32_t j = sb; j < se; ++j) dd += (stack[j] >> 31) ? 1 : -1;
         for (uint32_t j = pb; j < pe; ++j) {
-            if (pseq[j] >= n_prods) { err = "production id out of range"; return 4; }
             dv += arity[pseq[j]] - 1;
             if (pterm[pseq[j]] >= 0) ++nt;
         }

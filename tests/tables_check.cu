@@ -48,11 +48,19 @@ static bool sentinels() {
            refusal(section(1, 1, 5, 2, 5, 4)) == no && refusal(section(0, 1, 5, 2, 3, 0x40000000u)) == no;
 }
 
+// productions that no pair takes are read all the same
+static bool productions() {
+    const std::string no = "production id out of range";
+    return refusal(section(1, 1, 5, 2, 3, 4, {0, 0})).empty() && refusal(section(1, 1, 5, 2, 3, 4, {0, 1})) == no &&
+           refusal(section(1, 1, 5, 2, 3, 4, {0x7fffffffu, 0})) == no;
+}
+
 int main(int argc, char** argv) {
     const char* name = argc > 1 ? argv[1] : "";
     bool ok = false;
     if (!strcmp(name, "arity")) ok = arity(0) && !arity(1) && !arity(64) && !arity(INT32_MAX);
     if (!strcmp(name, "sentinels")) ok = sentinels();
+    if (!strcmp(name, "productions")) ok = productions();
     if (ok) printf("ok\n");
     return ok ? 0 : 1;
 }

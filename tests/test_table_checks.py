@@ -21,7 +21,7 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("case", ["arity", "sentinels"])
+@pytest.mark.parametrize("case", ["arity", "sentinels", "productions"])
 def test_tables_that_no_front_end_makes(exe, case):
     room = 4 << 30
     out = subprocess.run([exe, case], capture_output=True, text=True, timeout=120,
