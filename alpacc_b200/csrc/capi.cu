@@ -790,12 +790,14 @@ int lex3_grid(alp_ctx* ctx, const Lex3Run& r, const void* k, int threads, size_t
 }
 
 int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long* d_off, long long nd, int sentinels,
-                 void* term, void* start, void* end, long long cap, uint8_t* valid, Lex3Run& r, bool wide = true) {
+                 void* term, void* start, void* end, long long cap, uint8_t* valid, Lex3Run& r, bool walk = true) {
     r.tiles = (n + LX_TILE - 1) / LX_TILE;
     r.wide = (n + LX_WIDE - 1) / LX_WIDE;
     r.chunks = (n + LX_CHUNK - 1) / LX_CHUNK;
-    // units of the state scan: 64 bytes, or single chunks where no walk follows
-    r.units = wide ? (r.chunks + 1) / 2 : r.chunks;
+    // units of the state scan: 64 bytes, or single chunks where no walk follows (the fused token
+    // pass, the speculative lexer), which then reserves no token records either: 80 bytes a chunk
+    // (144 where the initial state ends empty tokens) of some 90 in all
+    r.units = walk ? (r.chunks + 1) / 2 : r.chunks;
     r.stiles = (r.units + ls_tile(scan_g(ctx)) - 1) / ls_tile(scan_g(ctx));
     r.nd = nd;
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -807,9 +809,9 @@ int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long
     r.o_td = o_c + al(2 * (size_t)r.chunks + 64);
     r.o_ccs = r.o_td + al(8 * (size_t)r.tiles);
     const size_t o_r = r.o_ccs + al(8 * ((size_t)r.tiles / LT_CHUNK + 2));
-    const size_t o_x = o_r + al(16 * (size_t)r.chunks + 64);
-    const size_t o_us = o_x + al(2 * (size_t)lw_more(ctx->l3.slots) * r.chunks + 64);
-    const size_t sbytes = o_us + al((size_t)r.units + 64);
+    const size_t o_x = o_r + (walk ? al(16 * (size_t)r.chunks + 64) : 0);
+    const size_t o_us = o_x + (walk ? al(2 * (size_t)lw_more(ctx->l3.slots) * r.chunks + 64) : 0);
+    const size_t sbytes = o_us + (walk ? al((size_t)r.units + 64) : 0);
     int rc;
     if ((rc = grow(ctx, ctx->scratch, sbytes))) return rc;
     uint8_t* base = reinterpret_cast<uint8_t*>(ctx->scratch.p);
@@ -824,10 +826,10 @@ int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long
     a.n_units = r.units;
     a.unit_f = reinterpret_cast<uint16_t*>(base + o_f);
     a.chunk_s = base + o_s;
-    a.unit_s = wide ? base + o_us : a.chunk_s;
+    a.unit_s = walk ? base + o_us : a.chunk_s;
     a.chunk_c = reinterpret_cast<uint16_t*>(base + o_c);
-    a.chunk_r = base + o_r;
-    a.chunk_x = reinterpret_cast<uint16_t*>(base + o_x);
+    a.chunk_r = walk ? base + o_r : nullptr;
+    a.chunk_x = walk ? reinterpret_cast<uint16_t*>(base + o_x) : nullptr;
     a.tile_cs = reinterpret_cast<unsigned long long*>(base + o_cs);
     a.lb_vec = reinterpret_cast<uint32_t*>(base + o_vec);
     a.res = reinterpret_cast<AlpResult*>(base);
@@ -3744,7 +3746,8 @@ static int spec3_lex(alp_ctx* ctx, const uint16_t* wbf, const float* wf32, int n
             return rc;
         cap = (int64_t)(ctx->out[1].bytes / 8);
         Lex3Run r;
-        if ((rc = lex3_prepare(ctx, d_in, n, nullptr, 1, 0, ctx->out[0].p, ctx->out[1].p, ctx->out[2].p, cap, dvalid, r)))
+        if ((rc = lex3_prepare(ctx, d_in, n, nullptr, 1, 0, ctx->out[0].p, ctx->out[1].p, ctx->out[2].p, cap, dvalid, r,
+                               false)))
             return rc;
         SpecArgs sa;
         memset(&sa, 0, sizeof sa);
