@@ -126,9 +126,9 @@ struct alp_ctx {
     int32_t* h_ring = nullptr;
     cudaEvent_t ev_ring[RING_SLOTS] = {};
     HostPool* pool = nullptr;
-    // when set (alp_set_output_alloc): the caller's allocator for the outputs of alp_lex,
-    // alp_parse, alp_parse_tokens and the batch entry points
-    alp_alloc_fn alloc_fn = nullptr;
+    // the caller's allocator (alp_set_output_alloc), and in alloc_fn during the entry points
+    // that take it (OutputScope): the others keep their device outputs in the context
+    alp_alloc_fn alloc_set = nullptr, alloc_fn = nullptr;
     void* alloc_user = nullptr;
     void* alloc_off = nullptr;    // of a batch: where the allocator wants the documents' offsets
     void* alloc_valid = nullptr;  // and their validity (null: left in the context's buffers)
@@ -370,6 +370,15 @@ int grow(alp_ctx* ctx, DevBuf& b, size_t bytes) {
     b.bytes = want;
     return ALP_OK;
 }
+
+// In an entry point whose outputs the caller's allocator gives: alp_lex, alp_parse,
+// alp_parse_tokens, alp_pre_productions, alp_lex_batch, alp_parse_batch.  Calls that go through
+// the same code for something else (host buffers, state labels, shards, tuning) have none.
+struct OutputScope {
+    alp_ctx* ctx;
+    explicit OutputScope(alp_ctx* c) : ctx(c) { ctx->alloc_fn = ctx->alloc_set; }
+    ~OutputScope() { ctx->alloc_fn = nullptr; }
+};
 
 // Outputs of n elements each from the caller's allocator (`count` pointers).
 int alloc_outputs(alp_ctx* ctx, long long n, void** ptrs, int count) {
@@ -2183,19 +2192,17 @@ int alp_tune_parse(alp_ctx* ctx, const uint8_t* d_in, int64_t n, int reps, char*
     long long nodes0 = -1;
     // median ms of `reps` calls with the context's current tuning
     auto measure = [&](double* ms) -> int {
-        int64_t *pp, *ps, *pe;
-        uint32_t* pt;
-        uint8_t* pk;
+        ParseOut o{};
         int64_t nn = 0;
         int valid = 0;
-        int r = alp_parse(ctx, d_in, n, &pp, &pt, &pk, &ps, &pe, &nn, &valid);  // warm-up
+        int r = parse_core(ctx, d_in, n, &o, 0, 1, &nn, &valid);  // warm-up
         if (r) return r;
         if (nodes0 < 0) nodes0 = nn;
         if (nn != nodes0) return fail(ctx, ALP_ERR_CUDA, "tuning variants disagree on the node count");
         std::vector<float> t;
         for (int i = 0; i < reps; ++i) {
             if (cudaEventRecord(e0, ctx->stream) != cudaSuccess) return fail(ctx, ALP_ERR_CUDA, "event record failed");
-            if ((r = alp_parse(ctx, d_in, n, &pp, &pt, &pk, &ps, &pe, &nn, &valid))) return r;
+            if ((r = parse_core(ctx, d_in, n, &o, 0, 1, &nn, &valid))) return r;
             if (cudaEventRecord(e1, ctx->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess)
                 return fail(ctx, ALP_ERR_CUDA, "event record failed");
             float x = 0;
@@ -2580,13 +2587,13 @@ static int tokens_out(alp_ctx* ctx, long long m, uint32_t** d_term, int64_t** d_
 
 int alp_set_output_alloc(alp_ctx* ctx, alp_alloc_fn fn, void* user) {
     if (!ctx) return ALP_ERR_ARG;
-    ctx->alloc_fn = fn;
+    ctx->alloc_set = fn;
     ctx->alloc_user = user;
     return ALP_OK;
 }
 
-int alp_lex(alp_ctx* ctx, const uint8_t* d_in, int64_t n, uint32_t** d_term, int64_t** d_start,
-            int64_t** d_end, int64_t* n_tok, int* valid) {
+static int lex_call(alp_ctx* ctx, const uint8_t* d_in, int64_t n, uint32_t** d_term, int64_t** d_start,
+                    int64_t** d_end, int64_t* n_tok, int* valid) {
     int rc = check_in(ctx, d_in, n, true);
     if (rc) return rc;
     if (!d_term || !d_start || !d_end || !n_tok || !valid) return fail(ctx, ALP_ERR_ARG, "null output");
@@ -2620,6 +2627,13 @@ int alp_lex(alp_ctx* ctx, const uint8_t* d_in, int64_t n, uint32_t** d_term, int
     return tokens_out(ctx, *valid ? *n_tok : 0, d_term, d_start, d_end);
 }
 
+int alp_lex(alp_ctx* ctx, const uint8_t* d_in, int64_t n, uint32_t** d_term, int64_t** d_start,
+            int64_t** d_end, int64_t* n_tok, int* valid) {
+    if (!ctx) return ALP_ERR_ARG;
+    OutputScope scope(ctx);
+    return lex_call(ctx, d_in, n, d_term, d_start, d_end, n_tok, valid);
+}
+
 int alp_lex_host(alp_ctx* ctx, const uint8_t* h_in, int64_t n, uint32_t* h_term, int64_t* h_start,
                  int64_t* h_end, int64_t cap, int64_t* n_tok, int* valid) {
     int rc = check_in(ctx, h_in, n, true);
@@ -2633,7 +2647,7 @@ int alp_lex_host(alp_ctx* ctx, const uint8_t* h_in, int64_t n, uint32_t* h_term,
     int64_t *ds, *de;
     ctx->last_h2d = n;
     ctx->last_d2h = 0;
-    rc = alp_lex(ctx, (const uint8_t*)ctx->tmp[0].p, n, &dt, &ds, &de, n_tok, valid);
+    rc = lex_call(ctx, (const uint8_t*)ctx->tmp[0].p, n, &dt, &ds, &de, n_tok, valid);
     if (rc) return rc;
     if (*n_tok > cap) return fail(ctx, ALP_ERR_CAPACITY, "host token buffer too small");
     const size_t M = (size_t)*n_tok;
@@ -3469,6 +3483,7 @@ int alp_parse(alp_ctx* ctx, const uint8_t* d_in, int64_t n, int64_t** d_parent, 
     if (!d_parent || !d_tag || !d_kind || !d_start || !d_end || !n_node || !valid)
         return fail(ctx, ALP_ERR_ARG, "null output");
     CK(cudaSetDevice(ctx->device));
+    OutputScope scope(ctx);
     ParseOut o{};
     rc = parse_core(ctx, d_in, n, &o, 0, 1, n_node, valid);
     if (rc) return rc;
@@ -3523,6 +3538,7 @@ int alp_parse_tokens(alp_ctx* ctx, const uint32_t* d_term, const int64_t* d_tsta
         return fail(ctx, ALP_ERR_ARG, "null output");
     if (!ctx->has_parser) return fail(ctx, ALP_ERR_MODE, "these tables have no parser");
     CK(cudaSetDevice(ctx->device));
+    OutputScope scope(ctx);
     PosHead head;
     int rc = tokens_in(ctx, d_term, d_tstart, d_tend, m, &head);
     if (rc) return rc;
@@ -3548,6 +3564,7 @@ int alp_pre_productions(alp_ctx* ctx, const uint32_t* d_term, int64_t m, uint32_
     if (!d_prod || !n_prod || !valid) return fail(ctx, ALP_ERR_ARG, "null output");
     if (!ctx->has_parser) return fail(ctx, ALP_ERR_MODE, "these tables have no parser");
     CK(cudaSetDevice(ctx->device));
+    OutputScope scope(ctx);
     PosHead head;
     int rc = tokens_in(ctx, d_term, nullptr, nullptr, m, &head);
     if (rc) return rc;
@@ -3572,7 +3589,7 @@ int alp_lex_states(alp_ctx* ctx, const uint8_t* d_in, int64_t n, uint8_t* d_stat
     int64_t m;
     int valid;
     ctx->state_out = d_states;
-    rc = alp_lex(ctx, d_in, n, &t, &st, &en, &m, &valid);
+    rc = lex_call(ctx, d_in, n, &t, &st, &en, &m, &valid);
     ctx->state_out = nullptr;
     return rc;
 }
@@ -3794,7 +3811,7 @@ static int spec3_lex(alp_ctx* ctx, const uint16_t* wbf, const float* wf32, int n
         const long long rounds = ctx->h_res->aux[0], reruns = ctx->h_res->aux[1], first = ctx->h_res->aux[2];
         if (rounds < 0) {
             // predictions too poor for the fix-up rounds: the plain lexer decides
-            rc = alp_lex(ctx, d_in, n, d_term, d_start, d_end, n_tok, valid);
+            rc = lex_call(ctx, d_in, n, d_term, d_start, d_end, n_tok, valid);
             if (stats) { stats[0] = K; stats[1] = first; stats[2] = reruns; stats[3] = -1; }
             return rc;
         }
@@ -3904,7 +3921,7 @@ int alp_lex_speculative(alp_ctx* ctx, const uint16_t* wbf, const float* wf32, in
             if (rounds > 64) break;  // predictions too poor: the plain scan decides
         }
         if (rounds > 64) {
-            rc = alp_lex(ctx, d_in, n, d_term, d_start, d_end, n_tok, valid);
+            rc = lex_call(ctx, d_in, n, d_term, d_start, d_end, n_tok, valid);
             if (stats) { stats[0] = K; stats[1] = first; stats[2] = reruns; stats[3] = -1; }
             return rc;
         }
@@ -3952,6 +3969,7 @@ int alp_lex_batch(alp_ctx* ctx, const uint8_t* d_in, const int64_t* d_off, int64
         return fail(ctx, ALP_ERR_ARG, "bad batch arguments");
     if (!ctx->has_lexer) return fail(ctx, ALP_ERR_MODE, "these tables have no lexer");
     CK(cudaSetDevice(ctx->device));
+    OutputScope scope(ctx);
     int64_t n = 0;
     CK(cudaMemcpyAsync(ctx->h_stage, d_off + n_docs, 8, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -4001,6 +4019,7 @@ int alp_parse_batch(alp_ctx* ctx, const uint8_t* d_in, const int64_t* d_off, int
         return fail(ctx, ALP_ERR_ARG, "bad batch arguments");
     if (!ctx->has_lexer || !ctx->has_parser) return fail(ctx, ALP_ERR_MODE, "these tables are not lexer+parser tables");
     CK(cudaSetDevice(ctx->device));
+    OutputScope scope(ctx);
     CK(cudaMemcpyAsync(ctx->h_stage, d_off + n_docs, 8, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     const int64_t n = ctx->h_stage[0];

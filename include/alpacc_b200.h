@@ -120,7 +120,8 @@ int alp_memcpy(alp_ctx* ctx, void* dst, const void* src, size_t bytes);
  * offsets to ptrs[ALP_ALLOC_OFF] and its validity to ptrs[ALP_ALLOC_VALID] where
  * these are set (they are null on entry).  A nonzero return ends the call with
  * ALP_ERR_CUDA.  It must not call back into the context.  A single input that is
- * rejected may get no call; a batch gets one whatever its documents' verdicts.  fn NULL: outputs are owned by the context again. */
+ * rejected may get no call; a batch gets one whatever its documents' verdicts.  No
+ * other entry point calls it.  fn NULL: outputs are owned by the context again. */
 enum { ALP_ALLOC_OFF = 5, ALP_ALLOC_VALID = 6, ALP_ALLOC_PTRS = 7 };
 typedef int (*alp_alloc_fn)(void* user, int64_t n, void** ptrs);
 int alp_set_output_alloc(alp_ctx* ctx, alp_alloc_fn fn, void* user);
