@@ -805,7 +805,7 @@ int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long
     r.chunks = (n + LX_CHUNK - 1) / LX_CHUNK;
     // units of the state scan: 64 bytes, or single chunks where no walk follows (the fused token
     // pass, the speculative lexer), which then reserves no token records either: 80 bytes a chunk
-    // (144 where the initial state ends empty tokens) of some 90 in all
+    // (144 where the initial state ends empty tokens) of some 86 in all
     r.units = walk ? (r.chunks + 1) / 2 : r.chunks;
     r.stiles = (r.units + ls_tile(scan_g(ctx)) - 1) / ls_tile(scan_g(ctx));
     r.nd = nd;
@@ -931,7 +931,9 @@ int lex3_tiles(alp_ctx* ctx, Lex3Run& r) {
 
 template <typename TermT, typename PosT>
 int lex3_emit(alp_ctx* ctx, Lex3Run& r, bool tiles_done = false) {
-    const void* k5 = r.walked ? (const void*)lex3_write_kernel<TermT, PosT> : (const void*)lex3_emit_kernel<TermT, PosT>;
+    const void* k5 = !r.walked ? (const void*)lex3_emit_kernel<TermT, PosT>
+                     : r.nd == 1 ? (const void*)lex3_write_kernel<TermT, PosT, true>
+                                 : (const void*)lex3_write_kernel<TermT, PosT, false>;
     const size_t sm = r.walked ? lex3_write_smem() : ctx->l3_emit_smem;
     unsigned g5;
     int rc;

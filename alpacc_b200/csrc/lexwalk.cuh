@@ -190,7 +190,10 @@ __global__ void __launch_bounds__(LX_THREADS, 6) lex3_walk_kernel(Lex3Args a, Le
 
 __host__ __device__ inline size_t lex3_write_smem() { return (size_t)(LX_THREADS / 32) * (2 * LW_WARP + 64 * 4); }
 
-template <typename TermT, typename PosT>
+// ONE: a single document, whose boundaries are the input's ends.  Its form has no searches for
+// documents, which leaves the registers to the token loop: 512 MiB take 500 us in it, 585 in
+// the form for several.
+template <typename TermT, typename PosT, bool ONE>
 __global__ void __launch_bounds__(LX_THREADS, 5) lex3_write_kernel(Lex3Args a, LexSeg sg) {
     const int S = a.t.S;
     __shared__ unsigned long long s_dmax;
@@ -208,11 +211,11 @@ __global__ void __launch_bounds__(LX_THREADS, 5) lex3_write_kernel(Lex3Args a, L
     if (tid < S) s_tok[tid] = a.t.tokinfo[tid];
     after_prior_kernel();
     const long long n = a.n;
-    const long long ND = sg.n_docs;
+    const long long ND = ONE ? 1 : sg.n_docs;
     // document holding position p of this tile: the largest d in [d0, dmax]
     // with off[d] <= p, from the shared offsets when the tile has few documents
     auto doc_of = [&](long long d0, long long dmax, long long p) -> long long {
-        if (dmax == d0) return d0;
+        if (ONE || dmax == d0) return d0;
         if (dmax - d0 < LX_DOCS) {
             int lo = 0, hi = (int)(dmax - d0);
             while (lo < hi) {
@@ -224,7 +227,7 @@ __global__ void __launch_bounds__(LX_THREADS, 5) lex3_write_kernel(Lex3Args a, L
         return doc_upper(sg.doc_off, d0, dmax, p);
     };
     auto base_of = [&](long long d0, long long dmax, long long d) -> long long {
-        return (dmax - d0 < LX_DOCS) ? (long long)s_doff[d - d0] : sg.doc_off[d];
+        return (ONE || dmax - d0 < LX_DOCS) ? (long long)s_doff[d - d0] : sg.doc_off[d];
     };
     TermT* o_term = reinterpret_cast<TermT*>(a.out_term);
     PosT* o_start = reinterpret_cast<PosT*>(a.out_start);
@@ -294,7 +297,7 @@ __global__ void __launch_bounds__(LX_THREADS, 5) lex3_write_kernel(Lex3Args a, L
         __syncthreads();
         long long dmax = d0;
         if (edges) {
-            dmax = (long long)s_dmax;
+            dmax = ONE ? 0 : (long long)s_dmax;
             heads = *reinterpret_cast<const uint2*>(s_head + 2 * tid);
             lasts = *reinterpret_cast<const uint2*>(s_last + 2 * tid);
         }
@@ -311,7 +314,12 @@ __global__ void __launch_bounds__(LX_THREADS, 5) lex3_write_kernel(Lex3Args a, L
             // documents that start or end in this thread's bytes: record by record and
             // boundary by boundary, in the order token before the byte, head, last token
             // (a head's own end flag, from an accepting initial state, comes after the head)
+            // The chunk's record i and the one after it are held, the next load in flight while a
+            // token is stored, and a head's documents follow from the one before: with a load for
+            // each test of a record and a search for each head 300,000 documents of one byte took
+            // 412 us here, 161 so (a second DFA walk 168); 40,000 of ten bytes 127 and 78 (63).
             uint32_t t = Xc + wc + ic - cnt, i = 0, h = 0, cur = cur0;
+            uint32_t r0 = record(c, 0), r1 = record(c, 1);
             long long doc = doc_of(d0, dmax, my);
             long long base = base_of(d0, dmax, doc);
             const unsigned long long hd = heads.x | ((unsigned long long)heads.y << 32), ls = lasts.x | ((unsigned long long)lasts.y << 32);
@@ -322,8 +330,8 @@ __global__ void __launch_bounds__(LX_THREADS, 5) lex3_write_kernel(Lex3Args a, L
                     st == ALP_NONE32 ? snone : (long long)st - base + pb, (long long)(at + end) - base + pb);
                 ++t;
             };
-            const uint32_t left[2] = {cnt0, cnt - cnt0};
-            uint32_t kept = 0;  // tokens of the current chunk so far
+            uint32_t left = cnt0;  // tokens of the current chunk to come
+            auto step = [&]() { r0 = r1; r1 = record(c + h, ++i + 1u); };
             for (int j = 0; j < lim;) {
                 // the next boundary at or after byte j, or the end of the chunk
                 const unsigned long long ev = (hd | ls) >> j;
@@ -332,21 +340,24 @@ __global__ void __launch_bounds__(LX_THREADS, 5) lex3_write_kernel(Lex3Args a, L
                 const bool bnd = b < cend;
                 const bool head = bnd && ((hd >> b) & 1ull), last = bnd && ((ls >> b) & 1ull);
                 const uint32_t bo = (uint32_t)(b - (int)h * LX_CHUNK);  // its offset in the chunk
-                auto next = [&]() { tok(record(c + h, i), h, (record(c + h, i) >> 5) & 31u); ++i; ++kept; };
+                auto next = [&]() { tok(r0, h, (r0 >> 5) & 31u); --left; step(); };
                 // a token ends before byte b itself (its last byte's own record comes after it)
                 auto at_b = [&]() {
-                    if (kept >= left[h] || ((record(c + h, i) >> 5) & 31u) != bo) return false;
-                    if (!last) return true;
-                    const uint32_t r2 = record(c + h, i + 1);
-                    return (r2 >> 10) != (LW_STOP >> 10) && ((r2 >> 5) & 31u) == bo;
+                    if (!left || ((r0 >> 5) & 31u) != bo) return false;
+                    return !last || ((r1 >> 10) != (LW_STOP >> 10) && ((r1 >> 5) & 31u) == bo);
                 };
-                while (kept < left[h] && ((record(c + h, i) >> 5) & 31u) < bo) next();
+                while (left && ((r0 >> 5) & 31u) < bo) next();
                 if (head) {
-                    // every document starting here (empty ones first, then the real one)
+                    // every document starting here (empty ones first, then the real one): past the
+                    // thread's first byte the ones right after the current document
                     const long long pos = my + b;
-                    doc = doc_of(d0, dmax, pos);
-                    long long dl = doc;  // empty documents that start here too
-                    while (dl > 0 && sg.doc_off[dl - 1] >= pos) --dl;
+                    long long dl = doc;
+                    if (b > 0) {
+                        dl = doc + 1;
+                        while (++doc < dmax && base_of(d0, dmax, doc + 1) <= pos) {}
+                    } else {
+                        while (dl > 0 && sg.doc_off[dl - 1] >= pos) --dl;
+                    }
                     base = pos;
                     for (long long e2 = dl; e2 <= doc; ++e2) {
                         sg.tok_off[e2] = t;
@@ -359,11 +370,12 @@ __global__ void __launch_bounds__(LX_THREADS, 5) lex3_write_kernel(Lex3Args a, L
                 }
                 if (bnd && at_b()) next();
                 if (last) {
-                    const uint32_t r = record(c + h, i++), ti = s_tok[r & 31u];
+                    const uint32_t ti = s_tok[r0 & 31u];
                     if (!(ti & TOK_IGNORE)) {
-                        tok(r, h, bo + 1u);
-                        ++kept;
+                        tok(r0, h, bo + 1u);
+                        --left;
                     }
+                    step();
                     sg.valid[doc] = (ti & TOK_ACCEPT) ? 1 : 0;
                     if (sent) put((long long)t + 2 * doc + 1, sg.sent_r, 0, 0);
                 }
@@ -371,8 +383,12 @@ __global__ void __launch_bounds__(LX_THREADS, 5) lex3_write_kernel(Lex3Args a, L
                 if (j >= LX_CHUNK && h == 0) {
                     h = 1;
                     i = 0;
-                    kept = 0;
+                    left = cnt - cnt0;
                     cur = cur1;
+                    if (lim > LX_CHUNK) {
+                        r0 = record(c + 1, 0);
+                        r1 = record(c + 1, 1);
+                    }
                 }
             }
         }
