@@ -1366,20 +1366,20 @@ int run_tree(alp_ctx* ctx, TreeArgs& t, bool one) {
 }
 
 int run_tree_escapes(alp_ctx* ctx, TreeArgs& t) {
-    const long long tiles = (t.L + PP_TILE - 1) / PP_TILE;
+    long long tiles = (t.L + PP_TILE - 1) / PP_TILE;
     mark(ctx, "start");
-    long long count = tiles;
-    int rc, split = tiles <= TR_LEVELS ? 8 : 1;
-    void* args[] = {&t, &count, &split};
     // Up to 1024 tiles (some 2 M positions) the searches read the one block's minima
-    // themselves, 4 KB a warp, and a tile has eight warps: without the launch of the levels and
-    // with more searches at once 4 MB of json take 133 us, not 139.
+    // themselves, 4 KB a warp: without the launch of the levels and with more searches at once
+    // 4 MB of json take 133 us, not 139.
     const bool levels = tiles > TR_LEVELS;
+    uint32_t head = levels ? 64 : 32;
+    void* args[] = {&t, &tiles, &head};
+    int rc;
     if (levels && (rc = launch_next(ctx, (const void*)tree_levels_kernel, (unsigned)(((tiles + 31) / 32 + 255) / 256), 256, 0,
                                     args)))
         return rc;
-    const long long g = (tiles * split + 7) / 8;
-    if ((rc = launch_next(ctx, (const void*)tree_escape_kernel, (unsigned)(g < 148 * 8 ? g : 148 * 8), 256, 0, args))) return rc;
+    const long long full = 8ll * ctx->sms;
+    if ((rc = launch_next(ctx, (const void*)tree_escape_kernel, (unsigned)std::min(tiles, full), 256, 0, args))) return rc;
     mark(ctx, levels ? "tree_levels+tree_escape" : "tree_escape_kernel");
     return ALP_OK;
 }
