@@ -447,7 +447,7 @@ class Grammar:
         """[tile shape, pair CTAs per SM, expand CTAs per SM, MLP kernel (0 tcgen05, 1 mma.sync),
         lexer token pass (0 fused, 1 walk with token records + tile scan + write pass),
         parser position pass (0 fused, 1 pair pass + tile-sum scan + expansion),
-        lexer state-scan chunks per lane (8, 16 or 32)]."""
+        lexer state-scan units (64 bytes; 32 in the fused pass) per lane (8, 16 or 32)]."""
         cfg = (ctypes.c_int32 * 7)()
         native().alp_tune_get(self.h, cfg, 7)
         return list(cfg)
@@ -455,7 +455,7 @@ class Grammar:
     def set_tuning(self, cfg: Sequence[int]) -> None:
         """Three values (launch shapes), four (and the MLP inference kernel),
         five (and the lexer's token pass), six (and the parser's position
-        pass) or seven (and the lexer state scan's chunks per lane)."""
+        pass) or seven (and the lexer state scan's units per lane)."""
         if len(cfg) not in (3, 4, 5, 6, 7):
             raise ValueError("tuning takes 3 to 7 values")
         c = (ctypes.c_int32 * len(cfg))(*cfg)

@@ -786,7 +786,7 @@ inline const void* scan_kernel_for(int g) {
     return (const void*)lex3_scan_kernel<16>;
 }
 
-// the state scan over the chunk endomorphisms, chunks per lane as tuned
+// the state scan over the unit endomorphisms, units per lane as tuned
 int lex3_scan(alp_ctx* ctx, Lex3Run& r);
 
 int lex3_grid(alp_ctx* ctx, const Lex3Run& r, const void* k, int threads, size_t smem, long long work, unsigned* g,
@@ -881,7 +881,7 @@ int lex3_prepare(alp_ctx* ctx, const uint8_t* d_in, long long n, const long long
     return ALP_OK;
 }
 
-// chunk endomorphisms
+// unit endomorphisms
 int lex3_fold(alp_ctx* ctx, Lex3Run& r) {
     unsigned g1;
     int rc;
@@ -899,7 +899,7 @@ int lex3_fold(alp_ctx* ctx, Lex3Run& r) {
     return ALP_OK;
 }
 
-// chunk endomorphisms -> chunk states -> chunk counts, masks and rows, and tile counts
+// unit endomorphisms -> unit states -> the walk: chunk states, counts and token records, and tile counts
 int lex3_front(alp_ctx* ctx, Lex3Run& r, bool folded = false) {
     unsigned g3;
     int rc;
@@ -1793,12 +1793,12 @@ int tokens_in(alp_ctx* ctx, const uint32_t* term, const int64_t* ts, const int64
     int rc;
     AlpResult* lex;
     if ((rc = grow(ctx, ctx->tmp[T_TTERM], (size_t)(m + 2) * 2 + 16)) || (rc = grow(ctx, ctx->tmp[T_TSTART], (size_t)(m + 2) * 4 + 16)) ||
-        (rc = grow(ctx, ctx->tmp[T_TEND], (size_t)(m + 2) * 4 + 16)) || (rc = positions_head(ctx, m + 2, &lex, &h->sy)))
+        (rc = grow(ctx, ctx->tmp[T_TEND], (size_t)(m + 2) * 4 + 16)) || (rc = device_limits(ctx)) || (rc = positions_head(ctx, m + 2, &lex, &h->sy)))
         return rc;
     h->base = reinterpret_cast<uint8_t*>(lex);
     h->ids = true;
-    const long long g = (m + 2 + 255) / 256;
-    tokens_in_kernel<<<(unsigned)(g < 148 * 8 ? g : 148 * 8), 256, 0, ctx->stream>>>(
+    const long long g = std::min((long long)(m + 2 + 255) / 256, 8ll * ctx->sms);
+    tokens_in_kernel<<<(unsigned)g, 256, 0, ctx->stream>>>(
         term, ts, te, m, (uint16_t*)ctx->tmp[T_TTERM].p, (uint32_t*)ctx->tmp[T_TSTART].p, (uint32_t*)ctx->tmp[T_TEND].p,
         ctx->pt.start, ctx->pt.end, (uint32_t)ctx->pt.T, std::min(ctx->pt.empty, (uint32_t)ctx->pt.T - 1u), lex,
         h->base + SC_VALID);
@@ -2248,7 +2248,7 @@ int alp_tune_parse(alp_ctx* ctx, const uint8_t* d_in, int64_t n, int reps, char*
         *field = arg;
         return ALP_OK;
     };
-    // lexer: the token pass's form, the state scan's chunks per lane
+    // lexer: the token pass's form, the state scan's units per lane
     {
         const int forms[] = {0, 1}, gs[] = {8, 16, 32};
         if ((rc = knob("lex_token_pass_split", &ctx->tune.lex_split, forms, 2)) ||
@@ -3311,7 +3311,7 @@ int alp_parse_shard_expand(alp_parse_shard* s, const int64_t* pre, int64_t pos_b
     if (!s || !pre || !n_node || !n_stair_nodes || !n_stair_brackets) return ALP_ERR_ARG;
     alp_ctx* ctx = s->ctx;
     CK(cudaSetDevice(ctx->device));
-    PosSums p;
+    PosSums p{};
     p.nodes = (uint32_t)pre[0]; p.brs = (uint32_t)pre[1]; p.depth = (int32_t)pre[2]; p.v = (int32_t)pre[3];
     p.terms = (uint32_t)pre[4]; p.heads = (uint32_t)pre[5]; p.hpos = (int32_t)pre[6]; p.cls = (uint32_t)pre[7];
     s->pos_base = pos_base;

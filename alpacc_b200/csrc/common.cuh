@@ -43,8 +43,6 @@ __device__ __forceinline__ void st_volatile64(unsigned long long* p, unsigned lo
     *reinterpret_cast<volatile unsigned long long*>(p) = v;
 }
 
-// Poll a 32-bit status word until its flag is not X.  Returns the word; on
-// timeout sets *err and returns a P word with value 0 so the caller finishes.
 // In a kernel launched by launch_next: past this point the kernel before it on the stream is
 // done and its writes are seen; the next kernel's blocks may come up behind this one's.  What
 // precedes it (the loads of the context's tables into shared memory, constant since the
@@ -56,6 +54,8 @@ __device__ __forceinline__ void after_prior_kernel() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Poll a 32-bit status word until its flag is not X.  Returns the word; on
+// timeout sets *err and returns a P word with value 0 so the caller finishes.
 __device__ __forceinline__ uint32_t wait32(const uint32_t* p, unsigned int* err) {
     uint32_t v = ld_volatile32(p);
     unsigned int ns = 32;

@@ -3,16 +3,16 @@
 // Same results as lex_seg_kernel (futhark/lexer.fut:73-172 per document),
 // split so that no step waits on another tile or on table lookups in L2:
 //
-//   lex3_fold_kernel   every 32-byte chunk -> its endomorphism id, folded with
-//                      the step table in shared memory (constant E+s after a
-//                      document head).  Two independent chunks per thread.
-//   lex3_scan_kernel   the composition scan over chunk endomorphisms.  With
+//   lex3_fold_kernel   every unit of 64 bytes (32 in the fused token pass) -> its
+//                      endomorphism id, folded with the step table in shared
+//                      memory (constant E+s after a document head).
+//   lex3_scan_kernel   the composition scan over unit endomorphisms.  With
 //                      S <= 32 one warp holds a whole function, lane s the
 //                      image of state s, so composing two functions is one
 //                      shuffle and a tile's aggregate is 32 bytes.  Lanes walk
-//                      the chunks of their warp through the apply table in
+//                      the units of their warp through the apply table in
 //                      shared memory; tiles chain through a decoupled look-back
-//                      on these vectors.  Output: the state entering each chunk.
+//                      on these vectors.  Output: the state entering each unit.
 //   lex3_walk_kernel   the token-end flags and ignore filter (futhark/lexer.fut:
 //                      103-107): each thread runs the DFA over two chunks from
 //                      their known states with a 256-column table whose entries
@@ -41,7 +41,7 @@ constexpr int LX_STAGE = 2048;                  // tokens one emit tile stages i
 constexpr int LS_WARPS = 8;
 constexpr int LS_BACK = 4;                      // tiles a look-back step of the state scan loads at once
 constexpr int LS_CHAINS = 4;                    // runs of units a warp follows side by side
-constexpr int LS_G = 16;                        // chunks per lane in the state scan (default; 8, 16 or 32)
+constexpr int LS_G = 16;                        // units per lane in the state scan (default; 8, 16 or 32)
 __host__ __device__ constexpr long long ls_tile(int g) { return (long long)LS_WARPS * 32 * g; }  // chunks per scan tile
 
 // ent entries: next state | flags.  Rows are LX_ROW entries apart so that
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(LX_THREADS, 4) lex3_fold_kernel(Lex3Args a, Le
 // One tile (a small call) 12.5 -> 8.5 us; 256 MiB stays at 51.
 template <int G>
 __global__ void __launch_bounds__(LS_WARPS * 32) lex3_scan_kernel(Lex3Args a) {
-    static_assert(G == 8 || G == 16 || G == 32, "chunks per lane");
+    static_assert(G == 8 || G == 16 || G == 32, "units per lane");
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t rows = (uint32_t)(a.t.E + a.t.S);
     uint8_t* s_app = smem;

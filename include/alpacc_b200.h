@@ -92,11 +92,12 @@ int alp_check_bounded_wait(alp_ctx* ctx);
  * predictions may differ where two logits are within rounding); with n >= 5,
  * cfg[4] the lexer's token pass (0: one fused pass that counts, looks back
  * over tiles and writes tokens; 1: a walk that counts and records tokens, a
- * tile scan and a write pass, the default); with n >= 6, cfg[5] the parser's position pass (0: one
- * fused pass that looks up the pairs, looks back over tiles and expands, sized
+ * tile scan and a write pass, the default); with n >= 6, cfg[5] the parser's
+ * position pass (0: one fused pass that looks up the pairs, looks back over tiles and expands, sized
  * from the previous parse on the context; 1: a pair pass and a scan of its
  * tile sums before the expansion, the default); with n >= 7, cfg[6] the lexer state
- * scan's chunks per lane (8, 16 or 32; 0 or 16 the default).  The tuner tries
+ * scan's units (64 bytes; 32 in the fused token pass) per lane (8, 16 or 32; 0
+ * or 16 the default).  The tuner tries
  * the lexer's knobs first, then the parser's.
  * alp_tune_parse times alp_parse on a sample (the median
  * of `reps` calls per candidate, CUDA events), one knob at a time, keeps the
