@@ -15,7 +15,7 @@
 // stream; the write pass by the latency of its record loads and its instruction stream.  For
 // 512 MiB of json (75 M tokens, 64-bit positions): walk 0.39 ms, write 0.50 ms, against 0.36 ms
 // for a counting walk and 0.68 ms for a second walk; the state scan over 64-byte units takes
-// 0.086 ms against 0.148 over chunks.  20,000 documents (245 MB): walk 0.24 and write 0.34 ms
+// 0.086 ms against 0.148 over chunks.  20,000 documents (245 MB): walk 0.24 and write 0.32 ms
 // against 0.26 and 0.47: a warp with a document boundary takes the same unrolled walk with two
 // tests a byte more, not a loop over the bytes of each boundary's thread.
 //
